@@ -7,28 +7,37 @@
 // row's off-diagonal entries in the reference's storage order; w[r] = rr *
 // dia (boost/numeric/mtl/operation/lower_trisolve.hpp:174-209,
 // upper_trisolve.hpp:161-176).  Only the schedule differs:
-//  - lane l of a warp owns the x-line j = 32 jb + l of plane k and runs its
-//    rows in x order, row i at step i + l: the x neighbour is the lane's own
-//    previous result (a register) and the y neighbour the lower lane's
-//    result of the previous step (a warp shuffle), so consecutive levels of
-//    a warp need no barrier;
-//  - the lane below lane 0 (the previous y-block) and the plane below run in
-//    other warps.  A CTA runs the NW warps of one tile (NW consecutive planes
-//    of one y-block, or NW consecutive y-blocks of a 2D grid) and hands
-//    results between them through shared-memory rings whose cells carry
-//    readiness in the value (the sentinel pattern marks an empty cell; the
-//    consumer empties a cell after reading it);
-//  - results of earlier tiles (other CTAs) are read from the output vector,
-//    which is all-sentinel before a sweep (each sweep resets the vector the
-//    next one writes), by two receiver warps that poll many steps at once
-//    and fill the same rings;
-//  - each warp's factor values, laid out step by step 32 lanes wide, stream
-//    into shared memory with bulk copies (TMA) several steps ahead, its
-//    right-hand sides with per-lane cp.async.
+//  - a lane owns one x-line and runs its rows in x order; a warp holds 8 x 4
+//    lines of neighbouring y and z (7-point) or 32 of neighbouring y
+//    (5-point), lane (a, b) running row i at step i + a + b: the x neighbour
+//    is the lane's own previous result (a register), the y and z neighbours
+//    are other lanes' results of the previous step (two warp shuffles);
+//  - a CTA runs the warps of one tile (2 x NW/2 warps, or NW along y).  A
+//    compute warp does nothing but the steps: it leaves its results in a
+//    shared ring, row by row of 32 lanes, and publishes its step count every
+//    kGridH steps; the warps at its upper y and z sides read their missing
+//    neighbours from that ring;
+//  - a helper warp per compute warp moves everything else: factor values by
+//    bulk copies (TMA), right-hand sides by cp.async and results from the
+//    ring to the output vector, both 8 consecutive rows of a line at a time
+//    (a lane per line would touch 32 sectors per instruction);
+//  - results on a tile's upper y and z sides also go, step by step, to a
+//    hand-off buffer in global memory (TriFactor::ghalo, all sentinel between
+//    sweeps), where the next tile's receiver warps poll them, fill a ring of
+//    the same form and put the sentinel back.
+// What bounds it: the dependency chain (nx + ny + nz steps and the hand-offs
+// between warps and tiles), not bytes; a step costs one shuffle, a row's
+// arithmetic and the shared-memory accesses that feed it.  Measured (one
+// B200, apply = L + U sweep, queued): FP32 ILU(0) 128^3 439 -> 230 us, 2048^2
+// 1,990 -> 773 us, FP64 128^3 773 -> 366 us against the previous kernel (one
+// warp per 32 lines and plane, every lane moving its own line's right-hand
+// sides, results and resets: 32 sectors per instruction, ~300 ns a step).
 // Tiles are taken through one ticket in an order in which every tile a tile
-// reads comes earlier, and a tile runs to its end on a running CTA, so the
-// waits end; every wait is still bounded (the context's spin_limit polls),
-// after which the kernel records a timeout and drains with zeros.
+// reads comes earlier, and a tile runs to its end on a running CTA.  Inside a
+// tile a warp waits on lower warps by at most two blocks of steps and on
+// upper ones only when a ring of four blocks is full, so the waits end; every
+// wait is still bounded (the context's spin_limit polls), after which the
+// kernel records a timeout and drains.
 // The same kernel computes the FP64 pivots of an ILU(0) or IC(0)
 // factorization of a grid-stencil pattern (OPK kGridILU0 / kGridIC0): a
 // row's pivot needs its earlier neighbours' pivots exactly as an L sweep's
@@ -37,17 +46,18 @@
 #pragma once
 #include "sweep.cuh"
 
+#include <climits>
+
 namespace mtlg {
 
-constexpr int kGridNB = 3;                  // staged factor blocks per compute warp
-constexpr int kGridG = 8;                   // steps per block (staged factor values, right-hand sides)
-constexpr int kGridRing = 32;               // steps per z / y ring (power of two)
-constexpr int kGridRhs = 32;                // right-hand-side ring (power of two, four blocks)
-constexpr int kGridRecvWarps = 2;           // receiver warps after the compute warps
-constexpr int kGridBatch = 16;              // steps per receiver batch
-static_assert(kGridRecvWarps * kGridBatch <= kGridRing, "receiver batches in flight must fit a ring");
+constexpr int kGridG = 8;                    // steps per staged block
+constexpr int kGridNB = 4;                   // staged blocks per warp (factor values and right-hand sides)
+constexpr int kGridRing = kGridG * kGridNB;  // rows of a ring (right-hand sides, results)
+constexpr int kGridH = 4;                    // steps between hand-offs inside a CTA
+constexpr int kGridRecvWarps = 2;            // receiver warps: z sides, y sides
+constexpr int kGridDiagRows = 8192;          // rows per tile of a factor without entries
 static_assert(kGridStepPad % kGridG == 0, "layout padding must hold whole staged blocks");
-static_assert(kGridRhs >= 3 * kGridG, "the right-hand-side ring holds the current block and two ahead");
+static_assert(kGridG % kGridH == 0, "hand-offs split a block evenly");
 
 // Row operations of the grid kernel: a triangular sweep, or the FP64 pivots
 // of an ILU(0) or IC(0) factorization (the same dependencies: a row's pivot
@@ -56,21 +66,30 @@ constexpr int kGridSweep = 0, kGridILU0 = 1, kGridIC0 = 2;
 // Slots per step (capacity): a sweep's entries and multiplier fit four; an
 // ILU(0) pivot reads its L entries, the neighbours' entries in its column and
 // its diagonal (up to seven).
-__host__ __device__ constexpr int grid_cap(int opk) { return opk == kGridILU0 ? 8 : 4; }
+__host__ __device__ constexpr int grid_cap(int opk) { return opk == kGridILU0 ? 7 : 4; }
 
-// Staged S elements per compute warp (kGridNB blocks of up to grid_cap slots).
-template <typename S, int OPK = kGridSweep>
-__host__ __device__ constexpr int grid_stage_elems()
-{
-    return kGridNB * kGridG * grid_cap(OPK) * 32;
-}
+// Elements between ring rows: 32 lanes and a pad that spreads the helper's
+// accesses (8 rows x 4 or 2 lines at once) over all banks.
+template <typename T>
+__host__ __device__ constexpr int grid_pitch() { return sizeof(T) == 4 ? 36 : 34; }
 
-// Dynamic shared memory of a k_sweep_grid CTA of nw compute warps.
+// Warp and tile shapes of a stencil with NS off-diagonal entries per row.
+template <int NW, int NS>
+struct GridShapeOf {
+    static constexpr int LY = NS == 3 ? kGridLY3 : 32, LZ = NS == 3 ? 32 / kGridLY3 : 1;   // lines per warp
+    static constexpr int WY = NS == 3 ? 2 : NW, WZ = NS == 3 ? NW / 2 : 1;                 // warps per tile
+    static constexpr int TY = LY * WY, TZ = LZ * WZ;                                       // lines per tile
+    static constexpr int SKEW = LY + LZ - 2;                                               // of a warp's last lane
+    static constexpr int ZCOLS = NS == 3 ? TY : 0;   // receiver ring columns of the z lines (first), then the y lines
+};
+
+// Dynamic shared memory of a k_sweep_grid CTA of nw compute warps: factor
+// blocks, right-hand-side ring and result ring per warp, the receiver's ring.
 template <typename T, typename S, int OPK = kGridSweep>
-__host__ __device__ inline int grid_smem_bytes(int nw)
+__host__ __device__ constexpr int grid_smem_bytes(int nw)
 {
-    return nw * (grid_stage_elems<S, OPK>() * int(sizeof(S)) + (kGridRhs + kGridRing) * 32 * int(sizeof(T)) +
-                 kGridRing * int(sizeof(T)));
+    const int ring = kGridRing * grid_pitch<T>() * int(sizeof(T));
+    return nw * (kGridRing * grid_cap(OPK) * 32 * int(sizeof(S)) + (OPK == kGridSweep ? 2 : 1) * ring) + ring;
 }
 
 // Slot orders the kernel runs (TriFactor::gperm): the farthest neighbour's
@@ -81,260 +100,559 @@ constexpr int kGridNear3 = 0 | (1 << 2) | (2 << 4);
 constexpr int kGridFar2 = 1 | (0 << 2);
 constexpr int kGridNear2 = 0 | (1 << 2);
 
-__device__ __forceinline__ long long grid_row(long long rp, int n, int rev) { return rev ? (long long)n - 1 - rp : rp; }
+// Values of one 16-byte group of a step's slots: sweeps of 7-point factors
+// keep a lane's four values together (one or two 16-byte shared loads a
+// step), the other layouts slot by slot.
+__host__ __device__ constexpr int grid_pack(int slots, int ssz) { return slots == 4 ? 16 / ssz : 1; }
+// Offset of a lane's slot q inside a step.
+__host__ __device__ inline int grid_slot(int pk, int q, int lane) { return (q / pk) * (32 * pk) + lane * pk + q % pk; }
 
-// Predicated stores (one instruction, no branch around it).
-__device__ __forceinline__ void st_slot_if(float* p, float v, bool c)
+// Hand-off rows between tiles: what a warp at a tile's upper z side leaves
+// at each step in its LY upper lines, [tile along z][unit along y][step][LY],
+// then at the upper y side, [tile along y][unit along z][step][LZ].
+inline size_t grid_halo_elems(int steps, int njb, int nkb, int ny, int nz, int ty, int tz, bool three)
 {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.volatile.shared.f32 [%0], %1;\n\t}" ::"r"(smem_u32(p)),
-                 "f"(v), "r"(int(c)));
-}
-__device__ __forceinline__ void st_slot_if(double* p, double v, bool c)
-{
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.volatile.shared.f64 [%0], %1;\n\t}" ::"r"(smem_u32(p)),
-                 "d"(v), "r"(int(c)));
-}
-__device__ __forceinline__ void st_relaxed_gpu_if(float* p, float v, bool c)
-{
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.relaxed.gpu.global.f32 [%0], %1;\n\t}" ::"l"(p), "f"(v),
-                 "r"(int(c)));
-}
-__device__ __forceinline__ void st_relaxed_gpu_if(double* p, double v, bool c)
-{
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.relaxed.gpu.global.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
-                 "r"(int(c)));
+    const int ly = three ? kGridLY3 : 32, lz = 32 / ly;
+    return ((three ? size_t((nz + tz - 1) / tz) * njb * ly : 0) + size_t((ny + ty - 1) / ty) * nkb * lz) * size_t(steps);
 }
 
-// Ring handoffs of a compute warp, warp-uniform: every lane takes part, a
-// lane without a cell to serve (act false) reads the CTA's dummy cell, which
-// always holds +0; the warp waits (bounded, then +0 and a timeout flag) until
-// every acting lane sees its value, then the acting lanes empty their cells.
-template <typename T>
-__device__ __noinline__ T grid_wait_take(T* p, T v, int* err, long long lim)
+// VN consecutive elements (16 bytes, or one) of a hand-off row, each checked on its own.
+template <int VN>
+__device__ __forceinline__ void ld_row(const float* p, float (&v)[VN])
+{
+    if constexpr (VN == 4) ld_relaxed_gpu4(p, v);
+    else v[0] = ld_relaxed_gpu(p);
+}
+template <int VN>
+__device__ __forceinline__ void ld_row(const double* p, double (&v)[VN])
+{
+    if constexpr (VN == 2)
+        asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "l"(p));
+    else v[0] = ld_relaxed_gpu(p);
+}
+__device__ __forceinline__ void st_sentinel_vec(void* p)
+{
+    asm volatile("st.global.v4.u32 [%0], {%1, %1, %1, %1};" ::"l"(p), "r"(0xFFFFFFFFu) : "memory");
+}
+
+// Shared memory by 32-bit address (the roles pick their rings at run time;
+// generic pointers would cost two registers and a generic access each).
+__device__ __forceinline__ void lds(unsigned a, float& v) { asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); }
+__device__ __forceinline__ void lds(unsigned a, double& v) { asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a)); }
+__device__ __forceinline__ void sts(unsigned a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v)); }
+__device__ __forceinline__ void sts(unsigned a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v)); }
+__device__ __forceinline__ void bulk_g2s_to(unsigned dst, const void* src, unsigned bytes, unsigned long long* bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void lds_vec(unsigned a, float* v)
+{
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(a));
+}
+__device__ __forceinline__ void lds_vec(unsigned a, double* v)
+{
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(a));
+}
+template <int VN>
+__device__ __forceinline__ void sts_row(unsigned a, const float (&v)[VN])
+{
+    if constexpr (VN == 4)
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]));
+    else sts(a, v[0]);
+}
+template <int VN>
+__device__ __forceinline__ void sts_row(unsigned a, const double (&v)[VN])
+{
+    if constexpr (VN == 2) asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v[0]), "d"(v[1]));
+    else sts(a, v[0]);
+}
+// Copies BYTES, or fills them with zeros (nothing is read then).
+template <int BYTES>
+__device__ __forceinline__ void cp_async_to(unsigned a, const void* gmem, bool copy)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(a), "l"(gmem), "n"(BYTES), "r"(copy ? BYTES : 0)
+                 : "memory");
+}
+
+// Step counts published inside the CTA: everything the publishing warp
+// stored before is visible to a warp that has read the count.
+__device__ __forceinline__ void grid_count(unsigned p, int v)
+{
+    asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int grid_read(unsigned p)
+{
+    int v;
+    asm volatile("ld.relaxed.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+    return v;
+}
+// After reading a count: what its writer stored before is visible from here on.
+__device__ __forceinline__ void grid_acquire() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
+// Waits until both counts reach their needs (bounded: on expiry, or when
+// another wait has expired, the warp goes on with whatever the rings hold).
+__device__ __forceinline__ void grid_wait(unsigned p, int need, unsigned p2, int need2, int* err, long long lim)
 {
     long long spins = 0;
-    while (__any_sync(0xffffffffu, is_sentinel(v))) {
+    while (__any_sync(0xffffffffu, grid_read(p) < need || grid_read(p2) < need2)) {
         if ((++spins & 255) == 0 && *(volatile int*)err) break;
         if (spins > (lim > 0 ? lim : kSpinLimit)) {
             atomicExch(err, 1);
             break;
         }
-        if (spins > 32) __nanosleep(32);   // a long wait leaves the issue slots to the producers
-        if (is_sentinel(v)) v = ld_slot(p);
     }
-    return is_sentinel(v) ? T(0) : v;
+    __syncwarp();
+    grid_acquire();
 }
-template <typename T>
-__device__ __forceinline__ T grid_take(T* cell, bool act, T* dummy, int* err, long long lim)
+// A staged block's barrier (own copies: a fixed bound, given up early once a
+// wait has expired; the helper waits for every copy before the tile ends).
+__device__ __forceinline__ void grid_bar_wait(unsigned long long* bar, unsigned parity, int* err)
 {
-    T* p = act ? cell : dummy;
-    T v = ld_slot(p);
-    if (__any_sync(0xffffffffu, is_sentinel(v))) v = grid_wait_take(p, v, err, lim);
-    st_slot_if(cell, sentinel_value<T>(), act);
-    return v;
-}
-// Fills ring cells once their previous values have been taken (same rules).
-template <typename T>
-__device__ __noinline__ void grid_wait_free(T* p, bool act, int* err, long long lim)
-{
-    long long spins = 0;
-    while (__any_sync(0xffffffffu, act && !is_sentinel(ld_slot(p)))) {
+    int spins = 0;
+    while (!mbar_try_wait(bar, parity)) {
         if ((++spins & 255) == 0 && *(volatile int*)err) return;
-        if (spins > (lim > 0 ? lim : kSpinLimit)) {
+        if (spins > 2 * int(kSpinLimit)) {
             atomicExch(err, 1);
             return;
         }
-        if (spins > 32) __nanosleep(32);
     }
 }
-template <typename T>
-__device__ __forceinline__ void grid_put(T* cell, bool act, T v, T* dummy, int* err, long long lim)
+// The thread's earlier cp.async copies arrive on the barrier when they land.
+__device__ __forceinline__ void cp_async_arrive(unsigned long long* bar)
 {
-    T* p = act ? cell : dummy;
-    if (__any_sync(0xffffffffu, act && !is_sentinel(ld_slot(p)))) grid_wait_free(p, act, err, lim);
-    st_slot_if(cell, v, act);
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// A compute warp's unit of one tile (pointers already offset by the lane
-// where the cell is per lane).
-template <typename T, typename S>
+// Shared-memory addresses of a tile's parts.
+struct GridSmem {
+    unsigned stage, rings;            // factor blocks, rings (per warp: results, right-hand sides; then the receiver's)
+    unsigned prog, vy, vz, inf;       // step counts: compute warps, the receivers' y and z rows, never-waiting
+    unsigned zero;                    // a cell that holds +0
+    unsigned long long* full;         // the staged blocks' barriers, kGridNB per warp
+    unsigned* blks;                   // staged blocks each warp has gone through before this tile
+};
+
+// What a compute warp works with (addresses of the lane's column where per lane).
+template <typename T>
 struct GridWarp {
-    const S* src;              // the unit's layout
-    S* stg;                    // its staged blocks (kGridNB)
-    unsigned long long* fb;    // their barriers
-    const T* vin;
-    T* vout;
-    T* vres;                   // nullptr: no reset vector
-    T* rr;                     // right-hand-side ring, this lane's column
-    T* zin;                    // incoming z ring, this lane's column
-    T* yin;                    // incoming y ring (lane 0)
-    T* zo;                     // outgoing z ring (the next plane's warp), this lane's column
-    T* yo;                     // outgoing y ring (the next y-block's warp; lane 31)
-    T* dummy;                  // the CTA's cell that always holds +0
-    long long rbase;           // r' of this lane's row i = 0
-    int n, nx, nsteps, lane;
-    bool lane_on, has_z, has_y, z_out, y_out;
+    unsigned stage, rhs, ring;        // staged factor blocks, right-hand-side ring, result ring
+    unsigned yin, zin;                // the y and z neighbours' columns (lanes at the warp's lower sides)
+    unsigned yp, zp;                  // bytes between their rows; no neighbour: 0, and yin / zin a cell that holds +0
+    unsigned yprog, zprog;            // step counts of those rings' writers
+    unsigned yfree, zfree;            // step counts of the own ring's readers
+    unsigned prog;                    // own step count
+    unsigned long long* full;
+    T* yhalo;                         // the lane's place in the hand-off row of step 0
+    T* zhalo;
+    unsigned blk;
+    int nx, nblk, lane;
+    bool lane_on;
+    bool yface, zface;                // the lane writes hand-off rows
     int* err;
     long long spin;
 };
 
-// The steps of one compute warp's unit: blocks of kGridG steps, each block's
-// factor values staged by a bulk copy kGridNB blocks ahead and its
-// right-hand sides by cp.async two blocks ahead; blocks where every lane has
-// a row at every step run without per-step validity tests.  NS entries per
-// row, FAR: the farthest neighbour's entry first (z, y, x; else x, y, z),
-// REV: rows counted from the end (U sweeps).
-template <typename T, typename S, int NS, bool FAR, bool REV, int OPK = kGridSweep>
-__device__ __forceinline__ void grid_warp_run(const GridWarp<T, S>& g, unsigned& phase)
+// Operands of kGridH steps of a lane: right-hand sides, neighbours' values
+// (lanes at the warp's lower sides), factor values.
+template <typename T, typename S, int SL>
+struct GridHalf {
+    T rr[kGridH], yv[kGridH], zv[kGridH];
+    S a[kGridH][SL];
+};
+
+// The steps of one compute warp's unit.  NS entries per row, FAR: the
+// farthest neighbour's entry first (z, y, x; else x, y, z).  While kGridH
+// steps run, the next ones' operands are loaded, a few per step (a burst of
+// shared loads would delay the shuffles behind it): factor values and
+// right-hand sides always, the neighbours' values when their writers' counts,
+// read at the start, already cover them; else they are waited for at the end.
+// A warp that has to wait falls behind until it no longer does, so the pace
+// is the chain of a step: shuffle, select, multiply, subtractions, multiply.
+// A sweep needs no validity tests: outside a lane's line factor values,
+// right-hand sides and so results are +0 (an absent neighbour).
+template <typename T, typename S, int NW, int NS, bool FAR, int OPK>
+__device__ __forceinline__ void grid_compute(const GridWarp<T>& g)
 {
+    typedef GridShapeOf<NW, NS> Sh;
     typedef typename std::conditional<(sizeof(S) > sizeof(T)), S, T>::type W;   // promoted type
-    constexpr int G = kGridG;
-    constexpr int SES = (OPK == kGridILU0 ? 2 * NS + 1 : NS + 1) * 32;   // S elements per step
-    constexpr int BE = G * grid_cap(OPK) * 32;                          // S elements per staged block (capacity)
-    constexpr bool SKEW = NS > 0;        // rows depend on the lane below: lane l runs row i at step i + l
-    const int lane = g.lane;
-    const int nblk = (g.nsteps + G - 1) / G;
-    const unsigned bbytes = unsigned(G * SES * int(sizeof(S)));
-    if (lane == 0)
-        for (int b = 0; b < kGridNB && b < nblk; ++b) {
-            mbar_expect_tx(&g.fb[b], bbytes);
-            bulk_g2s(g.stg + b * BE, g.src + size_t(b) * G * SES, bbytes, &g.fb[b]);
-        }
-    // right-hand sides of block m into their ring cells (one cp.async group)
-    auto fetch = [&](int m) {
-        if (OPK == kGridSweep && m < nblk) {
-            const int i0 = SKEW ? m * G - lane : m * G;
-            const long long r0 = g.rbase + i0;
-            const T* p = g.vin + (REV ? (long long)g.n - 1 - r0 : r0);
-            T* cell = g.rr + (((m * G) & (kGridRhs - 1)) << 5);
+    constexpr int G = kGridG, H = kGridH;
+    static_assert(G == 2 * H, "a block is two halves");
+    constexpr unsigned P = grid_pitch<T>() * sizeof(T);                         // bytes between ring rows
+    constexpr int SL = OPK == kGridILU0 ? 2 * NS + 1 : NS + 1;                  // slots per step
+    constexpr int PK = grid_pack(SL, int(sizeof(S)));
+    constexpr unsigned SB = 32 * SL * sizeof(S);                                // bytes per step
+    const int ly = g.lane % Sh::LY, lz = g.lane / Sh::LY;
+    const int total = g.nblk * G;
+    const bool ey = ly == 0, ez = lz == 0;
+    GridHalf<T, S, SL> A, B;
+    auto own = [&](GridHalf<T, S, SL>& d, int u, unsigned row, unsigned e) {   // step u's own operands
+        d.rr[u] = T(0);
+        if (OPK == kGridSweep) lds(g.rhs + row + u * P, d.rr[u]);
+        if constexpr (PK > 1) {
 #pragma unroll
-            for (int u = 0; u < G; ++u)
-                if (g.lane_on && i0 + u >= 0 && i0 + u < g.nx && r0 + u < g.n)
-                    cp_async_elem<sizeof(T)>(cell + (u << 5), REV ? p - u : p + u);
+            for (int k = 0; k < SL; k += PK) lds_vec(e + u * SB + k * (32 * unsigned(sizeof(S))), &d.a[u][k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < SL; ++k) lds(e + u * SB + k * (32 * unsigned(sizeof(S))), d.a[u][k]);
         }
-        cp_async_commit();
     };
-    fetch(0);
-    fetch(1);
-    T wx = T(0), wy = T(0);
-    for (int m = 0; m < nblk; ++m) {
-        const int s0 = m * G, b = m % kGridNB;
-        mbar_wait(&g.fb[b], (phase >> b) & 1u, g.err);
-        phase ^= 1u << b;
-        fetch(m + 2);
-        asm volatile("cp.async.wait_group 2;" ::: "memory");
-        const S* bk = g.stg + b * BE + lane;
-        const int c0 = s0 & (kGridRing - 1);   // ring cells of the block's steps: c0 + u (no wrap)
-        const T* rc = g.rr + (c0 << 5);
-        T* zi = g.zin + (c0 << 5);
-        T* zo = g.zo + (c0 << 5);
-        T* yi = g.yin + c0;
-        const int i0 = SKEW ? s0 - lane : s0;
-        const long long r0 = g.rbase + i0;
-        T* po = g.vout + (REV ? (long long)g.n - 1 - r0 : r0);
-        T* pr = g.vres ? g.vres + (REV ? (long long)g.n - 1 - r0 : r0) : nullptr;
-        auto steps = [&](auto edge) {
-            constexpr bool EDGE = decltype(edge)::value;
+    auto near = [&](GridHalf<T, S, SL>& d, int u, int s) {   // step u's neighbours' values (s: the half's first step)
+        lds(g.yin + unsigned((s + u + Sh::LY - 1) & (kGridRing - 1)) * g.yp, d.yv[u]);
+        d.zv[u] = T(0);
+        if (NS == 3) lds(g.zin + unsigned((s + u + Sh::LZ - 1) & (kGridRing - 1)) * g.zp, d.zv[u]);
+    };
+    auto wait_near = [&](int s) {   // the neighbours' values of the half at step s
+        grid_wait(g.yprog, min(s + H + Sh::LY - 1, total), g.zprog, min(s + H + Sh::LZ - 1, total), g.err, g.spin);
+    };
+    // result of the last step, and the y and z lower lanes' (+0 before a lane's first row)
+    T out = T(0), sy = T(0), sz = T(0);
+    T* yh = g.yhalo;
+    T* zh = g.zhalo;
+    auto half = [&](GridHalf<T, S, SL>& c, GridHalf<T, S, SL>& n, int m, int s0, unsigned enext, bool more) {
+        const int s1 = s0 + H;
+        const unsigned row = unsigned(s0 & (kGridRing - 1)) * P, rown = unsigned(s1 & (kGridRing - 1)) * P;
+        const int fy = grid_read(g.yprog), fz = grid_read(g.zprog), ry = grid_read(g.yfree), rz = grid_read(g.zfree);
+        T o[H];
 #pragma unroll
-            for (int u = 0; u < G; ++u) {
-                const int i = i0 + u;
-                bool valid = true;
-                if (EDGE) valid = g.lane_on && i >= 0 && i < g.nx && r0 + u < g.n;
-                T wz = T(0), wl = wy;
-                if (NS == 3 && g.has_z) wz = grid_take(zi + (u << 5), valid, g.dummy, g.err, g.spin);
-                if (NS >= 2 && g.has_y) {
-                    const T yv = grid_take(yi + u, valid && lane == 0, g.dummy, g.err, g.spin);
-                    wl = lane == 0 ? yv : wy;
-                } else if (NS >= 2) {
-                    wl = lane == 0 ? T(0) : wy;
+        for (int u = 0; u < H; ++u) {
+            const T wx = out, wy = ey ? c.yv[u] : sy, wz = ez ? c.zv[u] : sz;
+            const S* e = c.a[u];
+            T acc = OPK == kGridSweep ? c.rr[u] : T(e[SL - 1]);   // a pivot starts from a_ii
+            if constexpr (OPK == kGridILU0) {
+                // k_ilu0_factor on a grid stencil: per earlier neighbour k
+                // (ascending column) l = a_ik / u_kk (rounded), u_ii -= l a_ki
+                // (fused); L's entries and the other U entries do not change
+                if (NS == 3) acc = __fma_rn(-__dmul_rn(e[0], wz), e[NS], acc);
+                acc = __fma_rn(-__dmul_rn(e[NS - 2], wy), e[2 * NS - 2], acc);
+                acc = __fma_rn(-__dmul_rn(e[NS - 1], wx), e[2 * NS - 1], acc);
+            } else if constexpr (OPK == kGridIC0) {
+                // k_ic0_factor: d = a_ki / sqrt(u_kk) (rounded), u_ii -= d d
+                // (rounded product), per earlier neighbour k ascending
+                T d;
+                if (NS == 3) {
+                    d = __dmul_rn(e[0], wz);
+                    acc = __dsub_rn(acc, __dmul_rn(d, d));
                 }
-                const S* e = bk + u * SES;
-                T acc = OPK == kGridSweep ? rc[u << 5] : T(e[(SES / 32 - 1) * 32]);   // a pivot starts from a_ii
-                if constexpr (OPK == kGridILU0) {
-                    // k_ilu0_factor on a grid stencil: per earlier neighbour k
-                    // (ascending column) l = a_ik / u_kk (rounded), u_ii -= l a_ki
-                    // (fused); L's entries and the other U entries do not change
-                    if (NS == 3) {
-                        acc = __fma_rn(-__dmul_rn(e[0], wz), e[96], acc);
-                        acc = __fma_rn(-__dmul_rn(e[32], wl), e[128], acc);
-                        acc = __fma_rn(-__dmul_rn(e[64], wx), e[160], acc);
-                    } else if (NS == 2) {
-                        acc = __fma_rn(-__dmul_rn(e[0], wl), e[64], acc);
-                        acc = __fma_rn(-__dmul_rn(e[32], wx), e[96], acc);
-                    }
-                } else if constexpr (OPK == kGridIC0) {
-                    // k_ic0_factor: d = a_ki / sqrt(u_kk) (rounded), u_ii -= d d
-                    // (rounded product), per earlier neighbour k ascending
-                    if (NS == 3) {
-                        T d = __dmul_rn(e[0], wz);
-                        acc = __dsub_rn(acc, __dmul_rn(d, d));
-                        d = __dmul_rn(e[32], wl);
-                        acc = __dsub_rn(acc, __dmul_rn(d, d));
-                        d = __dmul_rn(e[64], wx);
-                        acc = __dsub_rn(acc, __dmul_rn(d, d));
-                    } else if (NS == 2) {
-                        T d = __dmul_rn(e[0], wl);
-                        acc = __dsub_rn(acc, __dmul_rn(d, d));
-                        d = __dmul_rn(e[32], wx);
-                        acc = __dsub_rn(acc, __dmul_rn(d, d));
-                    }
-                } else if constexpr (NS == 3) {
-                    if (FAR) {
-                        acc = sweep_step<T, S>(acc, e[0], wz);
-                        acc = sweep_step<T, S>(acc, e[32], wl);
-                        acc = sweep_step<T, S>(acc, e[64], wx);
-                    } else {
-                        acc = sweep_step<T, S>(acc, e[0], wx);
-                        acc = sweep_step<T, S>(acc, e[32], wl);
-                        acc = sweep_step<T, S>(acc, e[64], wz);
-                    }
-                } else if (NS == 2) {
-                    if (FAR) {
-                        acc = sweep_step<T, S>(acc, e[0], wl);
-                        acc = sweep_step<T, S>(acc, e[32], wx);
-                    } else {
-                        acc = sweep_step<T, S>(acc, e[0], wx);
-                        acc = sweep_step<T, S>(acc, e[32], wl);
-                    }
-                }
-                T out;
-                if constexpr (OPK == kGridILU0) out = unsentinel(T(__ddiv_rn(1.0, double(acc))));
-                else if constexpr (OPK == kGridIC0) out = unsentinel(T(__ddiv_rn(1.0, __dsqrt_rn(double(acc)))));
-                else out = unsentinel(T(W(acc) * W(e[NS * 32])));
-                if (EDGE) out = valid ? out : T(0);   // +0 outside the lane's line: an absent neighbour
-                st_relaxed_gpu_if(REV ? po - u : po + u, out, valid);
-                if (pr && valid) *(REV ? pr - u : pr + u) = sentinel_value<T>();
-                if (NS == 3 && g.z_out) grid_put(zo + (u << 5), valid, out, g.dummy, g.err, g.spin);
-                if (NS >= 2 && g.y_out)
-                    grid_put(g.yo + ((i) & (kGridRing - 1)), valid && lane == 31, out, g.dummy, g.err, g.spin);
-                if (SKEW) {
-                    wx = out;   // +0 before a lane's first row: its x neighbour is absent
-                    wy = __shfl_up_sync(0xffffffffu, out, 1);
-                }
+                d = __dmul_rn(e[NS - 2], wy);
+                acc = __dsub_rn(acc, __dmul_rn(d, d));
+                d = __dmul_rn(e[NS - 1], wx);
+                acc = __dsub_rn(acc, __dmul_rn(d, d));
+            } else if constexpr (FAR) {
+                if (NS == 3) acc = sweep_step<T, S>(acc, e[0], wz);
+                acc = sweep_step<T, S>(acc, e[NS - 2], wy);
+                acc = sweep_step<T, S>(acc, e[NS - 1], wx);
+            } else {
+                acc = sweep_step<T, S>(acc, e[0], wx);
+                acc = sweep_step<T, S>(acc, e[1], wy);
+                if (NS == 3) acc = sweep_step<T, S>(acc, e[2], wz);
             }
-        };
-        const bool inner = g.lane_on && i0 >= 0 && i0 + G <= g.nx && r0 + G <= g.n;
-        if (__all_sync(0xffffffffu, inner)) steps(std::integral_constant<bool, false>());
-        else steps(std::integral_constant<bool, true>());
-        // every lane is done with block m: refill its buffer with block m + kGridNB
+            if constexpr (OPK == kGridSweep) {
+                out = T(W(acc) * W(e[NS]));
+            } else {
+                // outside its line a lane's pivot is +0, as an absent neighbour's
+                const bool valid = g.lane_on && unsigned(s0 + u - ly - lz) < unsigned(g.nx);
+                if constexpr (OPK == kGridILU0) out = T(__ddiv_rn(1.0, double(acc)));
+                else out = T(__ddiv_rn(1.0, __dsqrt_rn(double(acc))));
+                out = valid ? out : T(0);
+            }
+            o[u] = out;
+            sy = __shfl_up_sync(0xffffffffu, out, 1);
+            if (NS == 3) sz = __shfl_up_sync(0xffffffffu, out, Sh::LY);
+            // (after the last block: stale shared memory, never used)
+            own(n, u, rown, enext);
+            if (u == 0) grid_acquire();
+            if (u > 0) near(n, u - 1, s1);
+            if (u == H - 1) near(n, u, s1);
+        }
+        const bool ok = fy >= min(s1 + H + Sh::LY - 1, total) && fz >= min(s1 + H + Sh::LZ - 1, total);
+        // the rows these results go to held those of a whole ring of steps ago
+        if (ry < s1 - kGridRing - (Sh::LY - 1) || rz < s1 - kGridRing - (Sh::LZ - 1))
+            grid_wait(g.yfree, s1 - kGridRing - (Sh::LY - 1), g.zfree, s1 - kGridRing - (Sh::LZ - 1), g.err, g.spin);
+#pragma unroll
+        for (int u = 0; u < H; ++u) sts(g.ring + row + u * P, o[u]);
         __syncwarp();
-        if (lane == 0 && m + kGridNB < nblk) {
-            mbar_expect_tx(&g.fb[b], bbytes);
-            bulk_g2s(g.stg + b * BE, g.src + size_t(m + kGridNB) * G * SES, bbytes, &g.fb[b]);
+        if (g.lane == 0) grid_count(g.prog, s1);
+        if (g.yface) {
+#pragma unroll
+            for (int u = 0; u < H; ++u) st_relaxed_gpu(yh + u * Sh::LZ, unsentinel(o[u]));
+        }
+        yh += H * Sh::LZ;
+        if (NS == 3) {
+            if (g.zface) {
+#pragma unroll
+                for (int u = 0; u < H; ++u) st_relaxed_gpu(zh + u * Sh::LY, unsentinel(o[u]));
+            }
+            zh += H * Sh::LY;
+        }
+        if (more && !ok) {
+            wait_near(s1);
+#pragma unroll
+            for (int u = 0; u < H; ++u) near(n, u, s1);
+        }
+    };
+    auto block = [&](int m) { return g.stage + ((g.blk + unsigned(m)) % kGridNB) * (G * SB); };
+    auto bar = [&](int m) {
+        const unsigned q = g.blk + unsigned(m);
+        grid_bar_wait(&g.full[q % kGridNB], (q / kGridNB) & 1u, g.err);
+    };
+    bar(0);
+#pragma unroll
+    for (int u = 0; u < H; ++u) own(A, u, 0u, block(0));
+    wait_near(0);
+#pragma unroll
+    for (int u = 0; u < H; ++u) near(A, u, 0);
+#pragma unroll 1
+    for (int m = 0; m < g.nblk; ++m) {
+        half(A, B, m, m * G, block(m) + H * SB, true);
+        const bool more = m + 1 < g.nblk;
+        if (more) bar(m + 1);
+        half(B, A, m, m * G + H, block(m + 1), more);
+    }
+}
+
+// A helper warp: thread t moves element t % 8 of lines t / 8 + 4 q, block by
+// block of a compute warp's steps (line l of block m: the rows of its steps
+// 8 m .. 8 m + 7, consecutive in x).
+template <typename T, typename S, int NW, int NS, bool REV, int OPK>
+__device__ __forceinline__ void grid_help(const S* src, unsigned stage, const T* vin, T* vout, unsigned rhs, unsigned ring,
+                                          unsigned prog, unsigned inf, unsigned long long* full, unsigned blk, int n, int nx,
+                                          int ny, int nz, int j0, int k0, int nblk, int lane, int* err, long long spin)
+{
+    typedef GridShapeOf<NW, NS> Sh;
+    constexpr int G = kGridG;
+    constexpr unsigned P = grid_pitch<T>() * sizeof(T);
+    constexpr int SL = OPK == kGridILU0 ? 2 * NS + 1 : NS + 1;
+    constexpr int BE = G * SL * 32;   // elements per staged block
+    const int xo = lane & 7, l0 = lane >> 3;
+    // the thread's element of line l0 + 4 q in block m: x = x0[q] + 8 m,
+    // vector index at[q] + (8 m or -8 m); kept in registers, since this
+    // warp's instructions bound the pace of its compute warp
+    int x0[8], at[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int a = (l0 + 4 * q) % Sh::LY, c = (l0 + 4 * q) / Sh::LY;
+        const int r = nx * (j0 + a + ny * (k0 + c)) + xo - a - c;
+        x0[q] = j0 + a < ny && k0 + c < nz ? xo - a - c : INT_MIN / 2;   // no such line: never inside
+        at[q] = REV ? n - 1 - r : r;
+    }
+    auto fetch = [&](int m) {
+        const unsigned c = blk + unsigned(m), b = c % kGridNB;
+        if (lane == 0) {
+            mbar_expect_tx(&full[b], unsigned(BE * int(sizeof(S))));
+            bulk_g2s_to(stage + b * unsigned(BE * sizeof(S)), src + size_t(m) * BE, unsigned(BE * int(sizeof(S))), &full[b]);
+        }
+        if (OPK == kGridSweep) {
+            const unsigned cell = rhs + (((m * G) & (kGridRing - 1)) + xo) * P + l0 * unsigned(sizeof(T));
+            const int x = m * G, o = REV ? -x : x;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const bool in = unsigned(x0[q] + x) < unsigned(nx);
+                cp_async_to<sizeof(T)>(cell + 4 * q * unsigned(sizeof(T)), vin + (in ? at[q] + o : 0), in);
+            }
+        }
+        cp_async_arrive(&full[b]);
+    };
+    for (int m = 0; m < kGridNB && m < nblk; ++m) fetch(m);
+#pragma unroll 1
+    for (int m = 0; m < nblk; ++m) {
+        grid_wait(prog, (m + 1) * G, inf, 0, err, spin);
+        const unsigned cell = ring + (((m * G) & (kGridRing - 1)) + xo) * P + l0 * unsigned(sizeof(T));
+        T v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) lds(cell + 4 * q * unsigned(sizeof(T)), v[q]);
+        __syncwarp();   // every lane has its results before the ring rows are released with the block
+        if (m + kGridNB < nblk) {
+            // block m's copies have landed (the compute warp has used them; an
+            // expired wait may have come here early)
+            const unsigned c = blk + unsigned(m);
+            mbar_wait(&full[c % kGridNB], (c / kGridNB) & 1u, err);
+            fetch(m + kGridNB);
+        }
+        const int x = m * G, o = REV ? -x : x;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (unsigned(x0[q] + x) < unsigned(nx)) vout[at[q] + o] = OPK == kGridSweep ? v[q] : unsentinel(v[q]);
+    }
+    // every copy of the tile has landed (also after an expired wait)
+    for (int m = max(0, nblk - kGridNB); m < nblk; ++m) {
+        const unsigned c = blk + unsigned(m);
+        mbar_wait(&full[c % kGridNB], (c / kGridNB) & 1u, err);
+    }
+}
+
+// A receiver warp: polls the hand-off rows of up to NG warps of earlier
+// tiles (`src`: rows of WD elements, one per step), puts each complete prefix
+// of rows into its ring (columns col + WD g) with the sentinel back in its
+// place, and publishes the count of rows there.  A thread holds VN elements
+// (16 bytes) of a row, so a group's poll is one coalesced load or a few.
+template <typename T, int WD, int NG>
+__device__ __forceinline__ void grid_receive(T* const (&src)[NG], int total, unsigned ring, int col, unsigned count,
+                                             unsigned reader, int reader_step, int slack, int lane, int* err, long long spin)
+{
+    constexpr int VN = WD * int(sizeof(T)) >= 16 ? 16 / int(sizeof(T)) : 1;   // elements per thread
+    constexpr int TR = WD / VN;                                              // threads per row
+    constexpr int RL = 32 / TR;                                              // rows per load
+    constexpr int NL = RL >= 16 ? 1 : 16 / RL;                               // loads per poll (at least 16 rows)
+    static_assert(VN == 1 ? WD == 1 : WD % VN == 0, "a row is whole vectors");
+    constexpr unsigned P = grid_pitch<T>() * sizeof(T);
+    const int tr = lane / TR, tc = (lane % TR) * VN;
+    int c[NG];   // rows delivered per group (warp-uniform)
+    unsigned left = 0;
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        c[g] = src[g] ? 0 : total;
+        if (src[g]) left |= 1u << g;
+    }
+    long long spins = 0;
+#pragma unroll 1
+    while (left) {
+        T v[NG][NL][VN];
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+#pragma unroll
+            for (int l = 0; l < NL; ++l) {
+                const int r = c[g] + l * RL + tr;
+                if (((left >> g) & 1u) && r < total) ld_row<VN>(src[g] + size_t(r) * WD + tc, v[g][l]);
+            }
+        bool moved = false;
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            if (!((left >> g) & 1u)) continue;
+            const int room = grid_read(reader + g * reader_step) + slack + kGridRing;   // rows below this are free
+            grid_acquire();
+            int rows = 0;
+            bool go = true;
+#pragma unroll
+            for (int l = 0; l < NL; ++l) {
+                const int r = c[g] + l * RL + tr;
+                bool ok = r < total && r < room;
+#pragma unroll
+                for (int e = 0; e < VN; ++e) ok = ok && !is_sentinel(v[g][l][e]);
+                // complete rows before the first that is not
+                const unsigned bad = ~__ballot_sync(0xffffffffu, ok);
+                const int got = !go ? 0 : bad ? (__ffs(bad) - 1) / TR : RL;
+                if (tr < got) {
+                    T* p = src[g] + size_t(r) * WD + tc;
+                    sts_row<VN>(ring + unsigned(r & (kGridRing - 1)) * P + unsigned(col + WD * g + tc) * unsigned(sizeof(T)), v[g][l]);
+                    if constexpr (VN > 1) st_sentinel_vec(p);
+                    else *p = sentinel_value<T>();
+                }
+                rows += got;
+                go = got == RL;
+            }
+            if (rows > 0) {
+                moved = true;
+                c[g] += rows;
+                __syncwarp();
+                if (lane == 0) grid_count(count + 4 * g, c[g]);
+                if (c[g] >= total) left &= ~(1u << g);
+            }
+        }
+        if (moved) continue;
+        if ((++spins & 255) == 0 && *(volatile int*)err) break;
+        if (spins > (spin > 0 ? spin : kSpinLimit)) {
+            if (lane == 0) atomicExch(err, 1);
+            break;
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    // after an expired wait nobody waits on these rows any more
+    if (left && lane == 0)
+        for (int g = 0; g < NG; ++g) grid_count(count + 4 * g, INT_MAX);
+}
+
+// The roles of one tile's warps (NS and FAR from the factor).  Not inlined:
+// with the four variants in one body the compiler keeps values of all of
+// them alive (96 registers and 370 bytes of spills instead of 80 and none).
+template <typename T, typename S, int NW, int NS, bool FAR, bool REV, int OPK>
+__device__ __noinline__ void grid_tile(const TriFactor& F, int n, const T* vin, T* vout, int ty, int tz,
+                                          const GridSmem& sm, int warp, int lane, int* err, long long spin)
+{
+    typedef GridShapeOf<NW, NS> Sh;
+    constexpr unsigned P = grid_pitch<T>() * sizeof(T), TS = sizeof(T);
+    constexpr int SL = OPK == kGridILU0 ? 2 * NS + 1 : NS + 1;
+    constexpr unsigned RB = kGridRing * P;                              // bytes of a ring
+    constexpr unsigned RW = (OPK == kGridSweep ? 2 : 1) * RB;           // rings of one warp: results, right-hand sides
+    constexpr unsigned SE = kGridRing * grid_cap(OPK) * 32 * sizeof(S); // staged bytes of one warp
+    const int nx = F.gnx, ny = F.gny, nz = F.gnz, njb = F.gnjb, nkb = (nz + Sh::LZ - 1) / Sh::LZ;
+    const int nblk = F.gnsp / kGridG, total = F.gnsp;
+    const int ntz = NS == 3 ? (nz + Sh::TZ - 1) / Sh::TZ : 0;
+    T* zh = static_cast<T*>(F.ghalo);                                    // [tile along z][unit along y][step][LY]
+    T* yh = zh + size_t(ntz) * njb * total * Sh::LY;                     // [tile along y][unit along z][step][LZ]
+    const unsigned rring = sm.rings + NW * RW;   // the receivers' (z columns, then y columns)
+    if (warp == 2 * NW) {
+        if constexpr (NS == 3) {
+            T* src[Sh::WY];
+#pragma unroll
+            for (int a = 0; a < Sh::WY; ++a) {
+                const int ju = ty * Sh::WY + a;
+                src[a] = tz > 0 && ju < njb ? zh + (size_t(tz - 1) * njb + ju) * total * Sh::LY : nullptr;
+            }
+            grid_receive<T, Sh::LY, Sh::WY>(src, total, rring, 0, sm.vz, sm.prog, 4, Sh::LZ - 1, lane, err, spin);
+        }
+        return;
+    }
+    if (warp > 2 * NW) {
+        T* src[Sh::WZ];
+#pragma unroll
+        for (int a = 0; a < Sh::WZ; ++a) {
+            const int ku = tz * Sh::WZ + a;
+            src[a] = ty > 0 && ku < nkb ? yh + (size_t(ty - 1) * nkb + ku) * total * Sh::LZ : nullptr;
+        }
+        grid_receive<T, Sh::LZ, Sh::WZ>(src, total, rring, Sh::ZCOLS, sm.vy, sm.prog, 4 * Sh::WY, Sh::LY - 1, lane, err, spin);
+        return;
+    }
+    const int w = warp % NW, wy = w % Sh::WY, wz = w / Sh::WY;
+    const int ju = ty * Sh::WY + wy, ku = tz * Sh::WZ + wz;
+    if (ju >= njb || ku >= nkb) return;
+    const int j0 = ju * Sh::LY, k0 = ku * Sh::LZ;
+    const unsigned blk = sm.blks[w], ring = sm.rings + w * RW;
+    if (warp >= NW) {
+        const S* src = static_cast<const S*>(F.gdata) + (size_t(ku) * njb + ju) * size_t(F.gnsp) * size_t(SL) * 32;
+        grid_help<T, S, NW, NS, REV, OPK>(src, sm.stage + w * SE, vin, vout, ring + RB, ring, sm.prog + 4 * w,
+                                          sm.inf, sm.full + w * kGridNB, blk, n, nx, ny, nz, j0, k0, nblk, lane, err, spin);
+        return;
+    }
+    const int ly = lane % Sh::LY, lz = lane / Sh::LY, j = j0 + ly, k = k0 + lz;
+    GridWarp<T> g;
+    constexpr int PK = grid_pack(SL, int(sizeof(S)));
+    g.stage = sm.stage + w * SE + lane * unsigned(PK * sizeof(S));
+    g.rhs = ring + RB + lane * TS;
+    g.ring = ring + lane * TS;
+    const bool has_y = ju > 0, has_z = NS == 3 && ku > 0;
+    g.yprog = !has_y ? sm.inf : wy > 0 ? sm.prog + 4 * (w - 1) : sm.vy + 4 * wz;
+    g.yin = !has_y ? sm.zero : wy > 0 ? ring - RW + (Sh::LY - 1 + Sh::LY * lz) * TS : rring + (Sh::ZCOLS + wz * Sh::LZ + lz) * TS;
+    g.zprog = !has_z ? sm.inf : wz > 0 ? sm.prog + 4 * (w - Sh::WY) : sm.vz + 4 * wy;
+    g.yp = has_y ? P : 0u;
+    g.zin = !has_z ? sm.zero : wz > 0 ? ring - Sh::WY * RW + (Sh::LY * (Sh::LZ - 1) + ly) * TS : rring + (wy * Sh::LY + ly) * TS;
+    g.zp = has_z ? P : 0u;
+    g.yfree = wy + 1 < Sh::WY && ju + 1 < njb ? sm.prog + 4 * (w + 1) : sm.inf;
+    g.zfree = wz + 1 < Sh::WZ && ku + 1 < nkb ? sm.prog + 4 * (w + Sh::WY) : sm.inf;
+    g.prog = sm.prog + 4 * w;
+    g.full = sm.full + w * kGridNB;
+    g.lane_on = j < ny && k < nz;
+    g.yface = wy == Sh::WY - 1 && ju + 1 < njb && ly == Sh::LY - 1;
+    g.zface = NS == 3 && wz == Sh::WZ - 1 && ku + 1 < nkb && lz == Sh::LZ - 1;
+    g.yhalo = yh + (size_t(ty) * nkb + ku) * total * Sh::LZ + lz;
+    g.zhalo = zh + (size_t(tz) * njb + ju) * total * Sh::LY + ly;
+    g.blk = blk;
+    g.nx = nx;
+    g.nblk = nblk;
+    g.lane = lane;
+    g.err = err;
+    g.spin = spin;
+    grid_compute<T, S, NW, NS, FAR, OPK>(g);
 }
 
 // One sweep over the grid tiles of a set of systems.  op.tasks: GroupTask
-// {sys, first unit along y, first plane, units along y per tile (jw)}; a
-// tile's warp q runs unit (first + q % jw, plane + q / jw).  Systems with z
-// neighbours are tiled with jw = 1 (the warps are consecutive planes).
+// {sys, tile along y, tile along z}; of a factor without entries (NS 0, its
+// multipliers in row order) {sys, first of kGridDiagRows rows / kGridDiagRows}.
 template <typename T, typename S, int NW, bool REV, int OPK = kGridSweep>
-__global__ void __launch_bounds__(32 * (NW + kGridRecvWarps)) k_sweep_grid(SetView sv, ChunkSweepOp op)
+__global__ void __launch_bounds__(32 * (2 * NW + kGridRecvWarps), 1) k_sweep_grid(SetView sv, ChunkSweepOp op)
 {
-    constexpr int NTH = 32 * (NW + kGridRecvWarps);
-    constexpr int SE = grid_stage_elems<S, OPK>();
+    constexpr int NTH = 32 * (2 * NW + kGridRecvWarps);
+    typedef typename std::conditional<(sizeof(S) > sizeof(T)), S, T>::type W;   // promoted type
     if (blockDim.x != unsigned(NTH) || op.which != int(REV)) {   // launch shape mismatch: report, never wait
         if (threadIdx.x == 0) atomicExch(sv.err, 1);
         return;
@@ -342,19 +660,29 @@ __global__ void __launch_bounds__(32 * (NW + kGridRecvWarps)) k_sweep_grid(SetVi
     extern __shared__ __align__(128) unsigned char grid_smem[];
     __shared__ __align__(8) unsigned long long full[NW * kGridNB];
     __shared__ int s_task, s_go;
-    __shared__ __align__(8) T grid_dummy;   // read by lanes without a ring cell to serve: always +0
-    S* stage = reinterpret_cast<S*>(grid_smem);
-    T* rhs_ring = reinterpret_cast<T*>(grid_smem + size_t(NW) * SE * sizeof(S));
-    T* zring = rhs_ring + NW * kGridRhs * 32;   // [warp][step % ring][lane]
-    T* yring = zring + NW * kGridRing * 32;     // [warp][row % ring]
+    __shared__ int prog[2 * NW + 4];   // step counts: compute warps, the receivers' y rows, their z rows; never waited on
+    __shared__ unsigned blks[NW];
+    __shared__ __align__(8) T zero;
+    constexpr int SE = kGridRing * grid_cap(OPK) * 32;
+    GridSmem sm;
+    sm.stage = smem_u32(grid_smem);
+    sm.rings = sm.stage + unsigned(NW * SE * int(sizeof(S)));
+    sm.prog = smem_u32(prog);
+    sm.vy = sm.prog + 4 * NW;
+    sm.vz = sm.vy + 4 * (NW + 1);   // 2D tiles: one y row per tile; 3D: NW / 2 y rows, two z rows
+    sm.inf = sm.vz + 4 * 2;
+    sm.zero = smem_u32(&zero);
+    sm.full = full;
+    sm.blks = blks;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-        grid_dummy = T(0);
-        for (int b = 0; b < NW * kGridNB; ++b) mbar_init(&full[b], 1);
+        // 32 cp.async arrivals of the helper's threads and its bulk copy
+        for (int b = 0; b < NW * kGridNB; ++b) mbar_init(&full[b], 33);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (tid < NW) blks[tid] = 0;
+    if (tid == 0) zero = T(0);
     __syncthreads();
-    unsigned phase = 0;   // compute warps: parity of the next wait on each of their staged blocks (bit b)
     for (;;) {
         if (tid == 0) {
             const int t = atomicAdd(op.ticket, 1);
@@ -362,7 +690,8 @@ __global__ void __launch_bounds__(32 * (NW + kGridRecvWarps)) k_sweep_grid(SetVi
             s_task = t;
             s_go = t < op.ntasks && !skip_system(sv.st[op.tasks[t].sys], op.skip) && !*(volatile int*)sv.err;
         }
-        for (int e = tid; e < NW * kGridRing * 33; e += NTH) zring[e] = sentinel_value<T>();   // z and y rings empty
+        if (tid >= 32 && tid < 32 + 2 * NW + 3) prog[tid - 32] = 0;
+        if (tid == 32 + 2 * NW + 3) prog[tid - 32] = INT_MAX;
         __syncthreads();
         const int t = s_task;
         if (t >= op.ntasks) break;
@@ -370,118 +699,31 @@ __global__ void __launch_bounds__(32 * (NW + kGridRecvWarps)) k_sweep_grid(SetVi
             const GroupTask gt = op.tasks[t];
             const SysDesc& d = sv.desc[gt.sys];
             const TriFactor& F = op.which == 0 ? d.L : d.U;
-            const int rev = int(REV);   // U: rows counted from the end
-            const int n = d.n, nx = F.gnx, ny = F.gny, nz = F.gnz, ns = F.gns, perm = F.gperm, dirs = F.gdirs;
-            const int nsteps = F.gnsteps, njb = F.gnjb;
-            const int jw = gt.pad, kw = NW / jw, ju0 = gt.pos0, k0 = gt.count;
+            const int n = d.n, ns = F.gns, ty = gt.pos0, tz = gt.count;
+            const T* vin = OPK == kGridSweep ? vptr<T>(d, op.in) : nullptr;
             T* vout = vptr<T>(d, op.out);
-            if (warp < NW) {
-                // ------------------------------------------------ compute warp
-                const int q = warp, qj = q % jw, qk = q / jw;
-                const int ju = ju0 + qj, k = k0 + qk;
-                if (ju < njb && k < nz) {
-                    const int j = 32 * ju + lane;
-                    GridWarp<T, S> g;
-                    const int slots = OPK == kGridILU0 ? 2 * ns + 1 : ns + 1;
-                    g.src = static_cast<const S*>(F.gdata) + (size_t(k) * njb + ju) * size_t(F.gnsp) * size_t(slots) * 32;
-                    g.stg = stage + size_t(q) * SE;
-                    g.fb = full + q * kGridNB;
-                    g.vin = vptr<T>(d, op.in);
-                    g.vout = vout;
-                    g.vres = op.reset != SLOT_NONE ? vptr<T>(d, op.reset) : nullptr;
-                    g.rr = rhs_ring + q * kGridRhs * 32 + lane;
-                    g.zin = zring + q * kGridRing * 32 + lane;
-                    g.yin = yring + q * kGridRing;
-                    g.zo = zring + (q + jw) * kGridRing * 32 + lane;   // used only when z_out
-                    g.yo = yring + (q + 1) * kGridRing;                // used only when y_out
-                    g.dummy = &grid_dummy;
-                    g.rbase = (long long)nx * ((long long)j + (long long)ny * k);
-                    g.n = n;
-                    g.nx = nx;
-                    g.nsteps = nsteps;
-                    g.lane = lane;
-                    g.lane_on = j < ny;
-                    g.has_z = (dirs & 4) && k > 0;
-                    g.has_y = (dirs & 2) && ju > 0;
-                    g.z_out = (dirs & 4) && qk + 1 < kw && k + 1 < nz;
-                    g.y_out = (dirs & 2) && qj + 1 < jw && ju + 1 < njb;
-                    g.err = sv.err;
-                    g.spin = sv.spin;
-                    if constexpr (OPK != kGridSweep) {
-                        // pivots: L's geometry, farthest neighbour first
-                        if (ns == 3) grid_warp_run<T, S, 3, true, false, OPK>(g, phase);
-                        else grid_warp_run<T, S, 2, true, false, OPK>(g, phase);
-                    } else if (ns == 3) {
-                        if (perm == kGridFar3) grid_warp_run<T, S, 3, true, REV>(g, phase);
-                        else grid_warp_run<T, S, 3, false, REV>(g, phase);
-                    } else if (ns == 2) {
-                        if (perm == kGridFar2) grid_warp_run<T, S, 2, true, REV>(g, phase);
-                        else grid_warp_run<T, S, 2, false, REV>(g, phase);
-                    } else {
-                        grid_warp_run<T, S, 0, false, REV>(g, phase);
-                    }
-                }
+            if (OPK == kGridSweep && ns == 0) {
+                const S* dia = static_cast<const S*>(F.gdata);
+                const int e = min(n, (ty + 1) * kGridDiagRows);
+                for (int r = ty * kGridDiagRows + tid; r < e; r += NTH) vout[r] = unsentinel(T(W(vin[r]) * W(dia[r])));
+            } else if (ns == 3) {
+                if (OPK != kGridSweep || F.gperm == kGridFar3)
+                    grid_tile<T, S, NW, 3, true, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin);
+                else
+                    grid_tile<T, S, NW, 3, false, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin);
             } else {
-                // ------------------------------------------------ receiver warps
-                // Receiver 0: the plane below the tile (jw == 1; lane l for
-                // lane l of the first plane's warp).  Receiver 1: the row
-                // below each warp's lane 0 (jw == 1: lane q for warp q;
-                // otherwise lane 0 for warp 0).  Each lane walks its own
-                // steps with a cursor: kGridBatch loads in flight, the ready
-                // prefix whose ring cells are free goes in, the rest waits
-                // for the next round, so no lane ever blocks another.
-                const int rw = warp - NW;
-                bool on;
-                long long base;     // r' of the lane's step 0 (Z: row i = s - lane; Y: row i = s)
-                T* cells;
-                int stride, c, end;
-                if (rw == 0) {
-                    on = jw == 1 && (dirs & 4) && k0 > 0 && 32 * ju0 + lane < ny;
-                    base = (long long)nx * ((long long)(32 * ju0 + lane) + (long long)ny * (k0 - 1)) - lane;
-                    cells = zring + lane;
-                    stride = 32;
-                    c = lane;
-                    end = min(nsteps, lane + nx);
-                } else {
-                    const int yk = jw == 1 ? k0 + lane : k0;
-                    on = rw == 1 && (dirs & 2) && ju0 > 0 && (jw == 1 ? (lane < kw && yk < nz) : lane == 0);
-                    base = (long long)nx * ((long long)(32 * ju0 - 1) + (long long)ny * yk);
-                    cells = yring + (jw == 1 ? lane : 0) * kGridRing;
-                    stride = 1;
-                    c = 0;
-                    end = nx;
-                }
-                if (!on) end = c;
-                const long long lim = sv.spin > 0 ? sv.spin : kSpinLimit;
-                long long spins = 0;
-                while (__any_sync(0xffffffffu, c < end)) {
-                    T v[kGridBatch];
-#pragma unroll
-                    for (int u = 0; u < kGridBatch; ++u)
-                        v[u] = c + u < end ? ld_relaxed_gpu(vout + grid_row(base + c + u, n, rev)) : sentinel_value<T>();
-                    int adv = 0;
-                    bool go = true;
-#pragma unroll
-                    for (int u = 0; u < kGridBatch; ++u) {
-                        T* cell = cells + ((c + u) & (kGridRing - 1)) * stride;
-                        go = go && c + u < end && !is_sentinel(v[u]) && is_sentinel(ld_slot(cell));
-                        st_slot_if(cell, v[u], go);
-                        adv += go ? 1 : 0;
-                    }
-                    c += adv;
-                    if (__any_sync(0xffffffffu, adv > 0)) continue;
-                    if ((++spins & 255) == 0 && *(volatile int*)sv.err) break;
-                    if (spins > lim) {
-                        atomicExch(sv.err, 1);
-                        break;
-                    }
-                    __nanosleep(op.sleep_ns > 0 ? op.sleep_ns : 64);
-                }
-                // after an expired wait: +0 into the cells still owed, so the compute warps drain
-                for (; c < end; ++c) {
-                    T* cell = cells + (c & (kGridRing - 1)) * stride;
-                    st_slot_if(cell, T(0), is_sentinel(ld_slot(cell)));
-                }
+                if (OPK != kGridSweep || F.gperm == kGridFar2)
+                    grid_tile<T, S, NW, 2, true, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin);
+                else
+                    grid_tile<T, S, NW, 2, false, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin);
+            }
+            __syncthreads();   // every warp has read its block count
+            if (tid < NW && ns > 0) {
+                // the blocks its warp went through keep the barriers' parity
+                const int wyn = ns == 3 ? 2 : NW;
+                const int lz = ns == 3 ? 32 / kGridLY3 : 1, wzn = ns == 3 ? NW / 2 : 1;
+                const int ju = ty * wyn + tid % wyn, ku = tz * wzn + tid / wyn;
+                if (ju < F.gnjb && ku < (F.gnz + lz - 1) / lz) blks[tid] += unsigned(F.gnsp / kGridG);
             }
         }
         __syncthreads();
@@ -499,8 +741,41 @@ __global__ void __launch_bounds__(32 * (NW + kGridRecvWarps)) k_sweep_grid(SetVi
 // lmul: ILU(0) factorized on the grid (A's values in `src`): L's entries are
 // a_rc times the inverse pivot of c, as k_ilu0_factor forms them.
 struct GridFillGeom {
-    int n, nx, ny, nz, ns, perm, skew, nsteps, nsp, njb;
+    int n, nx, ny, nz, ns, perm, nsp, njb;
+    int pk;   // grid_pack of the layout's slots
 };
+// Element e of a grid layout with `slots` slots per step: its slot, its row
+// r' (counted from the sweep's start) and the row's grid coordinates; false
+// for padding.  (A factor without entries holds its multipliers in row order.)
+struct GridElem {
+    int q, i, j, k;
+    long long r;
+};
+__host__ __device__ inline bool grid_elem(const GridFillGeom& g, int slots, long long e, GridElem& o)
+{
+    const int ly = g.ns == 3 ? kGridLY3 : 32;
+    const int w = int(e % (32 * slots)), in = w % (32 * g.pk);   // place in the step, in its group of pk slots
+    const int lane = in / g.pk;
+    o.q = w / (32 * g.pk) * g.pk + in % g.pk;
+    const long long rest = e / (32 * slots);
+    const int s = int(rest % g.nsp);
+    const long long u = rest / g.nsp;
+    const int a = lane % ly, b = lane / ly;
+    o.i = s - a - b;
+    o.j = int(u % g.njb) * ly + a;
+    o.k = int(u / g.njb) * (32 / ly) + b;
+    o.r = o.i + (long long)g.nx * (o.j + (long long)g.ny * o.k);
+    return o.i >= 0 && o.i < g.nx && o.j < g.ny && o.k < g.nz;
+}
+// The layout element of row r' and slot q.
+__host__ __device__ inline long long grid_elem_of(const GridFillGeom& g, int slots, long long r, int q)
+{
+    const int ly = g.ns == 3 ? kGridLY3 : 32, lz = 32 / ly;
+    const int i = int(r % g.nx), j = int((r / g.nx) % g.ny), k = int(r / ((long long)g.nx * g.ny));
+    const long long u = (long long)(k / lz) * g.njb + j / ly;
+    const int a = j % ly, b = k % lz;
+    return (u * g.nsp + i + a + b) * slots * 32 + grid_slot(g.pk, q, a + ly * b);
+}
 constexpr int kGridFillILU = 0, kGridFillIC = 1;
 __global__ void k_fill_grid_csr(long long nent, GridFillGeom g, int lower, int kind, int unit, int lmul,
                                 const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ src,
@@ -508,23 +783,24 @@ __global__ void k_fill_grid_csr(long long nent, GridFillGeom g, int lower, int k
 {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nent;
          e += (long long)gridDim.x * blockDim.x) {
-        const int lane = int(e & 31);
-        long long rest = e >> 5;
-        const int q = int(rest % (g.ns + 1));
-        rest /= (g.ns + 1);
-        const int s = int(rest % g.nsp);
-        const long long u = rest / g.nsp;
-        const int ju = int(u % g.njb), k = int(u / g.njb);
-        const int i = g.skew ? s - lane : s, j = 32 * ju + lane;
-        const long long rpr = i + (long long)g.nx * (j + (long long)g.ny * k);
+        GridElem o;
+        bool in;
+        if (g.ns == 0) {
+            o.q = 0;
+            o.r = lower ? e : g.n - 1 - e;
+            in = e < g.n;
+        } else {
+            in = grid_elem(g, g.ns + 1, e, o);
+        }
+        const int q = o.q;
         double v = 0.0;
-        if (s < g.nsteps && i >= 0 && i < g.nx && j < g.ny && rpr < g.n) {
-            const int r = lower ? int(rpr) : int(g.n - 1 - rpr);
+        if (in) {
+            const int r = lower ? int(o.r) : int(g.n - 1 - o.r);
             if (q == g.ns) {
                 v = unit ? 1.0 : inv_dia[r];
             } else {
                 const int d = (g.perm >> (2 * q)) & 3;
-                const bool present = d == 0 ? i > 0 : d == 1 ? j > 0 : k > 0;
+                const bool present = d == 0 ? o.i > 0 : d == 1 ? o.j > 0 : o.k > 0;
                 if (present) {
                     const long long off = d == 0 ? 1 : d == 1 ? g.nx : (long long)g.nx * g.ny;
                     const int c = int(lower ? r - off : r + off);
@@ -556,23 +832,18 @@ __global__ void k_fill_grid_factor(long long nent, GridFillGeom g, int kind, con
     const int slots = kind == kGridILU0 ? 2 * g.ns + 1 : g.ns + 1;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nent;
          e += (long long)gridDim.x * blockDim.x) {
-        const int lane = int(e & 31);
-        long long rest = e >> 5;
-        const int q = int(rest % slots);
-        rest /= slots;
-        const int s = int(rest % g.nsp);
-        const long long u = rest / g.nsp;
-        const int ju = int(u % g.njb), k = int(u / g.njb);
-        const int i = g.skew ? s - lane : s, j = 32 * ju + lane;
-        const long long r = i + (long long)g.nx * (j + (long long)g.ny * k);
+        GridElem o;
+        const bool in = grid_elem(g, slots, e, o);
+        const int q = o.q;
         double v = 0.0;
-        if (s < g.nsteps && i >= 0 && i < g.nx && j < g.ny && r < g.n) {
+        if (in) {
+            const long long r = o.r;
             int row = int(r), col = int(r);   // q == slots - 1: the diagonal
             bool present = true;
             if (q < slots - 1) {
                 const int qd = q < g.ns ? q : q - g.ns;
                 const int d = (g.perm >> (2 * qd)) & 3;
-                present = d == 0 ? i > 0 : d == 1 ? j > 0 : k > 0;
+                present = d == 0 ? o.i > 0 : d == 1 ? o.j > 0 : o.k > 0;
                 const long long off = d == 0 ? 1 : d == 1 ? g.nx : (long long)g.nx * g.ny;
                 const int nb = int(r - off);
                 const bool toward = kind == kGridILU0 && q < g.ns;   // a_ik (row r, column nb); else a_ki
@@ -601,13 +872,10 @@ __global__ void k_flat_from_grid(int npos, const int* __restrict__ row_of, const
         const int r = row_of[p];
         if (r < 0) continue;
         const long long rpr = lower ? r : (long long)g.n - 1 - r;
-        const int i = int(rpr % g.nx), j = int((rpr / g.nx) % g.ny), k = int(rpr / ((long long)g.nx * g.ny));
-        const long long u = (long long)k * g.njb + j / 32;
-        const int lane = j & 31, s = g.skew ? i + lane : i;
         for (int e = rp[p]; e < rp[p + 1]; ++e) {
             const long long off = lower ? (long long)r - ci[e] : (long long)ci[e] - r;
             const int d = off == 1 ? 0 : off == g.nx ? 1 : 2;
-            const long long src = ((u * g.nsp + s) * (g.ns + 1) + rank[d]) * 32 + lane;
+            const long long src = grid_elem_of(g, g.ns + 1, rpr, rank[d]);
             if (ssz == 8) reinterpret_cast<double*>(val)[e] = reinterpret_cast<const double*>(gval)[src];
             else reinterpret_cast<float*>(val)[e] = reinterpret_cast<const float*>(gval)[src];
         }

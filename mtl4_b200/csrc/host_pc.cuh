@@ -47,6 +47,7 @@ struct TriDev {
     // stencil): geometry as in TriFactor, per element the value source and
     // pivot row (kept until the values are filled), the values (type S)
     int gnx = 0, gny = 0, gnz = 0, gns = 0, gperm = 0, gdirs = 0, gskew = 0, gnsteps = 0, gnsp = 0, gnjb = 0;
+    DBuf<unsigned char> ghalo[2];      // hand-off rows between tiles for FP64 [0] / FP32 [1] vectors (all sentinel)
     long long gnent = 0;
     bool grid_indices = true;   // false: values filled straight from the matrix's CSR (no gsrc / gmul)
     DBuf<int> gsrc, gmul;
@@ -419,7 +420,7 @@ struct ChunkSide {
 struct ChunkPlan {
     bool ok = false;
     ChunkSide side[2];           // L [0], U [1]
-    DBuf<GroupTask> tl, tu;      // grid sweeps: tiles {sys, first unit along y, first plane, jw}
+    DBuf<GroupTask> tl, tu;      // grid sweeps: tiles {sys, tile along y, tile along z}
     int ntl = 0, ntu = 0;
     bool grid = false;           // k_sweep_grid: every factor of the set has a grid layout
     int gnw = 0, gsmem = 0, gresident = 0;   // compute warps, dynamic shared memory, CTAs resident at once
@@ -583,10 +584,10 @@ inline int chunk_groups(const std::vector<int>& nch, int cl, std::vector<GroupTa
 // and U, or nulls for an unused slot), in groups (chunk_groups) of the
 // side's cluster size.  Not ok (flat sweeps) when a side's shape is not built
 // or its shared memory does not fit.
-// Grid-sweep launch shapes: NW compute warps (4 or 8) and two receiver warps.
+// Grid-sweep launch shapes: NW compute warps (4 or 8), their helpers and two receiver warps.
 template <typename T, typename S, int NW>
 struct GridShape {
-    static constexpr int THREADS = 32 * (NW + kGridRecvWarps);
+    static constexpr int THREADS = 32 * (2 * NW + kGridRecvWarps);
     static int init()
     {
         if (grid_smem_bytes<T, S>(NW) > kChunkSmemMax) return MTLG_OK;   // not built for this type pair
@@ -624,7 +625,7 @@ struct GridShape {
 constexpr int kGridFactorWarpsILU = 2, kGridFactorWarpsIC = 4;
 template <int OPK, int NW>
 struct GridFactorShape {
-    static constexpr int THREADS = 32 * (NW + kGridRecvWarps);
+    static constexpr int THREADS = 32 * (2 * NW + kGridRecvWarps);
     static int smem() { return grid_smem_bytes<double, double, OPK>(NW); }
     static int init()
     {
@@ -666,16 +667,32 @@ inline void with_grid_shape(int nw, Fn&& fn)
     else fn(GridShape<T, S, 4>());
 }
 
+// Tiles of a grid factor for nw compute warps, diagonal by diagonal (tile
+// along y + tile along z): a tile reads its two lower neighbours only, and
+// the tiles that can run together come together.
+inline void grid_tiles(const TriDev& F, int nw, int sys, std::vector<GroupTask>& out)
+{
+    if (F.gns == 0) {
+        for (int r = 0; r < F.n; r += kGridDiagRows) out.push_back(GroupTask{sys, r / kGridDiagRows, 0, 0});
+        return;
+    }
+    const bool three = F.gns == 3;
+    const int ty = three ? 2 * kGridLY3 : 32 * nw, tz = three ? 32 / kGridLY3 * (nw / 2) : 1;
+    const int nty = (F.gny + ty - 1) / ty, ntz = (F.gnz + tz - 1) / tz;
+    for (int d = 0; d < nty + ntz - 1; ++d)
+        for (int z = std::max(0, d - nty + 1); z <= std::min(d, ntz - 1); ++z) out.push_back(GroupTask{sys, d - z, z, 0});
+}
+
 // Grid-sweep plan of a set whose factors all have grid layouts: compute
-// warps (the context's grid_warps, else 8 where the shared memory fits,
-// else 4), and per side the tiles of every system, taken round-robin over
-// the systems (a system's tiles plane block by plane block, y-blocks
-// ascending inside: every tile a tile reads comes earlier).  Systems with z
-// neighbours tile NW planes of one y-block (jw = 1), the others NW y-blocks.
+// warps (the context's grid_warps where the shared memory fits, else 4), and per side the tiles of every system (grid_tiles), taken
+// round-robin over the systems: every tile a tile reads comes earlier.
 template <typename T, typename S>
 inline int plan_grid(mtlg_ctx* c, const std::vector<std::pair<const TriDev*, const TriDev*>>& f, ChunkPlan& pl)
 {
-    int nw = c->grid_warps > 0 ? c->grid_warps : 8;
+    // four compute warps: one per SM sub-partition (eight, with half the
+    // hand-offs between CTAs, share the shared-memory pipe: FP32 128^3 L
+    // sweep 103 us with four, 146 us with eight)
+    int nw = c->grid_warps > 0 ? c->grid_warps : 4;
     if (grid_smem_bytes<T, S>(nw) > kChunkSmemMax) nw = 4;
     if (grid_smem_bytes<T, S>(nw) > kChunkSmemMax) return MTLG_OK;
     int res = 0;
@@ -689,9 +706,7 @@ inline int plan_grid(mtlg_ctx* c, const std::vector<std::pair<const TriDev*, con
             if (!f[s].first) continue;
             const TriDev& F = w == 0 ? *f[s].first : *f[s].second;
             steps = std::max(steps, F.gnsteps);
-            const int jw = (F.gdirs & 4) ? 1 : nw, kw = nw / jw;
-            for (int k0 = 0; k0 < F.gnz; k0 += kw)
-                for (int j0 = 0; j0 < F.gnjb; j0 += jw) per[s].push_back(GroupTask{int(s), j0, k0, jw});
+            grid_tiles(F, nw, int(s), per[s]);
             most = std::max(most, per[s].size());
         }
         std::vector<GroupTask> g;
@@ -859,7 +874,6 @@ inline TriFactor tri_view(const TriDev& T)
         f.gns = T.gns;
         f.gperm = T.gperm;
         f.gdirs = T.gdirs;
-        f.gskew = T.gskew;
         f.gnsteps = T.gnsteps;
         f.gnsp = T.gnsp;
         f.gnjb = T.gnjb;
@@ -1059,7 +1073,7 @@ inline bool detect_grid(const RowLists& F, int n, bool lower, TriDev& T)
 // Grid layout of a factor whose pattern detect_grid accepted: per unit,
 // step, slot and lane the value source and pivot row of the element
 // (k_fill_grid fills the values after the factorization).
-inline int build_grid(mtlg_ctx* c, const RowLists& F, int n, bool lower, TriDev& T)
+inline int build_grid(mtlg_ctx* c, const RowLists& F, int n, bool lower, int ssz, TriDev& T)
 {
     T.gnx = 0;
     T.gnent = 0;
@@ -1072,12 +1086,12 @@ inline int build_grid(mtlg_ctx* c, const RowLists& F, int n, bool lower, TriDev&
         }
     }
     MTLG_TRACE(9161, "pc.grid_layout");
-    T.gnjb = (T.gny + 31) / 32;
-    T.gnsteps = T.gskew ? T.gnx + std::min(T.gny, 32) - 1 : T.gnx;
+    const int ly = T.gns == 3 ? kGridLY3 : 32, lz = 32 / ly;
+    T.gnjb = (T.gny + ly - 1) / ly;
+    T.gnsteps = T.gns ? T.gnx + std::min(T.gny, ly) - 1 + std::min(T.gnz, lz) - 1 : T.gnx;
     T.gnsp = (T.gnsteps + kGridStepPad - 1) / kGridStepPad * kGridStepPad;
-    const int se = (T.gns + 1) * 32;
-    const long long units = (long long)T.gnjb * T.gnz;
-    const long long nent = units * T.gnsp * se;
+    const long long units = (long long)T.gnjb * ((T.gnz + lz - 1) / lz);
+    const long long nent = T.gns ? units * T.gnsp * (T.gns + 1) * 32 : n;
     if (nent > (long long)INT32_MAX) {
         T.gnx = 0;
         return MTLG_OK;
@@ -1085,38 +1099,36 @@ inline int build_grid(mtlg_ctx* c, const RowLists& F, int n, bool lower, TriDev&
     T.gnent = nent;
     if (!T.grid_indices) return MTLG_OK;
     hvec<int> gsrc(static_cast<size_t>(nent)), gmul(static_cast<size_t>(nent));
-    const int nx = T.gnx, ny = T.gny, ns = T.gns, perm = T.gperm, skew = T.gskew, nsteps = T.gnsteps;
-    const long long nxy = (long long)nx * ny;
-    parallel_for(int(units), [&](int u) {
-        const int ju = u % T.gnjb, k = u / T.gnjb;
-        long long e = (long long)u * T.gnsp * se;
-        for (int s = 0; s < T.gnsp; ++s)
-            for (int q = 0; q <= ns; ++q)
-                for (int l = 0; l < 32; ++l, ++e) {
-                    const int i = skew ? s - l : s, j = 32 * ju + l;
-                    const long long rp = i + (long long)nx * (j + (long long)ny * k);
-                    if (s >= nsteps || i < 0 || i >= nx || j >= ny || rp >= n) {
-                        gsrc[e] = -1;
-                        gmul[e] = -1;
-                        continue;
-                    }
-                    const int r = lower ? int(rp) : int(n - 1 - rp);
-                    if (q == ns) {
-                        gsrc[e] = -2;
-                        gmul[e] = r;
-                        continue;
-                    }
-                    const int d = (perm >> (2 * q)) & 3;
-                    const long long off = d == 0 ? 1 : d == 1 ? nx : nxy;
-                    const long long col = lower ? r - off : r + off;
-                    gsrc[e] = -1;
-                    gmul[e] = -1;
-                    for (int f = F.rp[r]; f < F.rp[r + 1]; ++f)
-                        if (F.col[f] == col) {
-                            gsrc[e] = F.src[f];
-                            gmul[e] = F.mul[f];
-                        }
+    const int nx = T.gnx, ns = T.gns, perm = T.gperm;
+    const long long nxy = (long long)nx * T.gny;
+    const GridFillGeom geom = {n, T.gnx, T.gny, T.gnz, T.gns, T.gperm, T.gnsp, T.gnjb, grid_pack(T.gns + 1, ssz)};
+    constexpr long long kBlk = 1 << 16;
+    parallel_for(int((nent + kBlk - 1) / kBlk), [&](int blk) {
+        for (long long e = blk * kBlk; e < std::min(nent, (blk + 1) * kBlk); ++e) {
+            gsrc[e] = -1;
+            gmul[e] = -1;
+            GridElem o;
+            if (ns == 0) {
+                gsrc[e] = -2;
+                gmul[e] = int(e);
+                continue;
+            }
+            if (!grid_elem(geom, ns + 1, e, o)) continue;
+            const int r = lower ? int(o.r) : int(n - 1 - o.r);
+            if (o.q == ns) {
+                gsrc[e] = -2;
+                gmul[e] = r;
+                continue;
+            }
+            const int d = (perm >> (2 * o.q)) & 3;
+            const long long off = d == 0 ? 1 : d == 1 ? nx : nxy;
+            const long long col = lower ? r - off : r + off;
+            for (int f = F.rp[r]; f < F.rp[r + 1]; ++f)
+                if (F.col[f] == col) {
+                    gsrc[e] = F.src[f];
+                    gmul[e] = F.mul[f];
                 }
+        }
     });
     MTLG_TRY(T.gsrc.upload(c, gsrc.data(), gsrc.size()));
     MTLG_TRY(T.gmul.upload(c, gmul.data(), gmul.size()));
@@ -1125,7 +1137,7 @@ inline int build_grid(mtlg_ctx* c, const RowLists& F, int n, bool lower, TriDev&
 
 inline int build_tri(mtlg_ctx* c, RowLists&& F, int n, bool lower, TriDev& T, int chunk_rows, int ssz, bool defer_flat)
 {
-    MTLG_TRY(build_grid(c, F, n, lower, T));
+    MTLG_TRY(build_grid(c, F, n, lower, ssz, T));
     // a factor swept on its grid layout (values filled from the CSR) needs no
     // chunked layout; its flat entries come on first need (ensure_flat)
     const bool grid_only = T.gnx > 0 && !T.grid_indices;
@@ -1215,6 +1227,7 @@ struct mtlg_pc {
     TriDev L, U;
     DBuf<double> inv_dia;           // FP64 pivots (ILU: 1/u_ii, IC: 1/sqrt(u_ii))
     DBuf<unsigned char> tmp;        // sentinel-filled temporary (n x 8 bytes)
+    bool tmp_used = false;          // a grid sweep left values in tmp: flat sweeps need the sentinel back first
     DBuf<int> tickets;              // self-resetting work tickets
     DBuf<SysDesc> desc;
     DBuf<SysState> st;
@@ -1252,6 +1265,20 @@ inline int ensure_ypos(mtlg_ctx* c, TriDev& T, int f32)
     return fill_sentinel(c, T.ypos[f32].p, bytes);
 }
 
+// Hand-off rows of a grid factor for vectors of one type (sized for the
+// smallest tiles, those of four compute warps), all sentinel between sweeps.
+inline int ensure_ghalo(mtlg_ctx* c, TriDev& T, int f32)
+{
+    if (T.gnx == 0 || T.gns == 0 || !T.gval.p || T.ghalo[f32].p) return MTLG_OK;
+    const bool three = T.gns == 3;
+    const int lz = three ? 32 / kGridLY3 : 1;
+    const size_t bytes = grid_halo_elems(T.gnsp, T.gnjb, (T.gnz + lz - 1) / lz, T.gny, T.gnz, three ? 2 * kGridLY3 : 128,
+                                         2 * lz, three) *
+                         (f32 ? 4 : 8);
+    MTLG_TRY(T.ghalo[f32].alloc(c, bytes));
+    return fill_sentinel(c, T.ghalo[f32].p, bytes);
+}
+
 // Device views of a preconditioner's factors for vectors of one type: each
 // sweep publishes into its own position-ordered results and resets the
 // other factor's (the next sweep of the other kind reads them sentinel).
@@ -1259,6 +1286,10 @@ inline int pc_views(mtlg_pc* P, int f32, TriFactor& L, TriFactor& U)
 {
     L = tri_view(P->L);
     U = tri_view(P->U);
+    MTLG_TRY(ensure_ghalo(P->ctx, P->L, f32));
+    MTLG_TRY(ensure_ghalo(P->ctx, P->U, f32));
+    L.ghalo = P->L.ghalo[f32].p;
+    U.ghalo = P->U.ghalo[f32].p;
     if (L.chunk_rows > 0 && U.chunk_rows > 0) {
         MTLG_TRY(ensure_ypos(P->ctx, P->L, f32));
         MTLG_TRY(ensure_ypos(P->ctx, P->U, f32));
@@ -1279,9 +1310,12 @@ inline int pc_reset_sweep_state(mtlg_pc* P)
 {
     if (!P) return MTLG_OK;
     for (TriDev* T : {&P->L, &P->U})
-        for (int k = 0; k < 2; ++k)
+        for (int k = 0; k < 2; ++k) {
             if (T->ypos[k].p) MTLG_TRY(fill_sentinel(P->ctx, T->ypos[k].p, T->ypos[k].n));
+            if (T->ghalo[k].p) MTLG_TRY(fill_sentinel(P->ctx, T->ghalo[k].p, T->ghalo[k].n));
+        }
     if (P->tmp.p) MTLG_TRY(fill_sentinel(P->ctx, P->tmp.p, size_t(P->n) * 8));
+    P->tmp_used = false;
     return MTLG_OK;
 }
 
@@ -1333,7 +1367,7 @@ inline int fill_grid_values(mtlg_pc* P, TriDev& T, const double* srcvals, const 
     const int f32 = P->storage == MTLG_F32;
     MTLG_TRY(T.gval.alloc(c, size_t(T.gnent) * P->ssize()));
     if (!T.grid_indices) {
-        const GridFillGeom g = {T.n, T.gnx, T.gny, T.gnz, T.gns, T.gperm, T.gskew, T.gnsteps, T.gnsp, T.gnjb};
+        const GridFillGeom g = {T.n, T.gnx, T.gny, T.gnz, T.gns, T.gperm, T.gnsp, T.gnjb, grid_pack(T.gns + 1, int(P->ssize()))};
         const int kind = P->kind == MTLG_PC_IC0 ? kGridFillIC : kGridFillILU;
         k_fill_grid_csr<<<launch_grid(T.gnent), 256, 0, c->stream>>>(T.gnent, g, T.lower ? 1 : 0, kind, unit,
                                                                    P->grid_factored ? 1 : 0, P->A->rp.p, P->A->ci.p,
@@ -1411,7 +1445,8 @@ inline int ensure_flat(mtlg_pc* P)
         MTLG_TRY(T->dia.alloc(c, size_t(std::max(T->npad, 1)) * P->ssize()));
         if (T->nnz && T->nch == 0 && T->gnx > 0 && T->gval.p) {
             // values from the grid layout
-            const GridFillGeom g = {T->n, T->gnx, T->gny, T->gnz, T->gns, T->gperm, T->gskew, T->gnsteps, T->gnsp, T->gnjb};
+            const GridFillGeom g = {T->n, T->gnx, T->gny, T->gnz, T->gns, T->gperm, T->gnsp, T->gnjb,
+                                    grid_pack(T->gns + 1, int(P->ssize()))};
             k_flat_from_grid<<<launch_grid(T->npad), 256, 0, c->stream>>>(T->npad, T->row_of.p, T->rp.p, T->ci.p, g,
                                                                           T->lower ? 1 : 0, T->gval.p, T->val.p,
                                                                           int(P->ssize()));
@@ -1462,10 +1497,10 @@ inline int grid_factorize(mtlg_pc* P, bool& done)
     if (res < 1) return MTLG_OK;
     MTLG_TRACE(9162, "pc.grid_factor");
     const int slots = kind == kGridILU0 ? 2 * L.gns + 1 : L.gns + 1;
-    const long long nent = (long long)L.gnjb * L.gnz * L.gnsp * slots * 32;
+    const long long nent = L.gnent / (L.gns + 1) * slots;
     DBuf<double> lay;
     MTLG_TRY(lay.alloc(c, size_t(nent)));
-    const GridFillGeom gg = {L.n, L.gnx, L.gny, L.gnz, L.gns, L.gperm, L.gskew, L.gnsteps, L.gnsp, L.gnjb};
+    const GridFillGeom gg = {L.n, L.gnx, L.gny, L.gnz, L.gns, L.gperm, L.gnsp, L.gnjb, grid_pack(slots, 8)};
     k_fill_grid_factor<<<launch_grid(nent), 256, 0, c->stream>>>(nent, gg, kind, P->A->rp.p, P->A->ci.p, P->A->v64.p,
                                                                  lay.p);
     c->launches++;
@@ -1481,16 +1516,22 @@ inline int grid_factorize(mtlg_pc* P, bool& done)
     d.L.gns = L.gns;
     d.L.gperm = L.gperm;
     d.L.gdirs = L.gdirs;
-    d.L.gskew = L.gskew;
     d.L.gnsteps = L.gnsteps;
     d.L.gnsp = L.gnsp;
     d.L.gnjb = L.gnjb;
     d.L.gdata = lay.p;
+    // hand-off rows of these tiles
+    DBuf<double> halo;
+    const bool three = L.gns == 3;
+    const int nkb = (L.gnz + (three ? 32 / kGridLY3 : 1) - 1) / (three ? 32 / kGridLY3 : 1);
+    const size_t nhalo = grid_halo_elems(L.gnsp, L.gnjb, nkb, L.gny, L.gnz, three ? 2 * kGridLY3 : 32 * nw,
+                                         three ? 32 / kGridLY3 * (nw / 2) : 1, three);
+    MTLG_TRY(halo.alloc(c, nhalo));
+    MTLG_TRY(fill_sentinel(c, halo.p, nhalo * sizeof(double)));
+    d.L.ghalo = halo.p;
     MTLG_CUDA(cudaMemcpyAsync(P->desc.p, &d, sizeof d, cudaMemcpyHostToDevice, c->stream));
     std::vector<GroupTask> tiles;
-    const int jw = L.gns == 3 ? 1 : nw, kw = nw / jw;
-    for (int k0 = 0; k0 < L.gnz; k0 += kw)
-        for (int j0 = 0; j0 < L.gnjb; j0 += jw) tiles.push_back(GroupTask{0, j0, k0, jw});
+    grid_tiles(L, nw, 0, tiles);
     DBuf<GroupTask> tl;
     MTLG_TRY(tl.upload(c, tiles.data(), tiles.size()));
     SetView sv;

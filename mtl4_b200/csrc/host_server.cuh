@@ -303,6 +303,9 @@ inline int srv_rebuild(mtlg_server* S, int e)
                 if (!pcs[s]) continue;
                 mtlg_pc* P = const_cast<mtlg_pc*>(pcs[s]);
                 MTLG_TRY(ensure_flat(P));
+                // grid sweeps of an earlier membership leave values in the L sweeps' output
+                const size_t zb = size_t(ss.h_desc[s].ws_stride) * vsize(ss.f32);
+                MTLG_TRY(fill_sentinel(c, static_cast<unsigned char*>(ss.h_desc[s].ws) + size_t(V_Z0) * zb, zb));
                 MTLG_TRY(pc_views(P, ss.f32, ss.h_desc[s].L, ss.h_desc[s].U));
                 ss.h_desc64[s].L = ss.h_desc[s].L;
                 ss.h_desc64[s].U = ss.h_desc[s].U;

@@ -92,7 +92,7 @@ struct SolveSet {
 };
 
 // After an expired device wait: the L sweeps' output (V_Z0) back to all
-// sentinel, as the flat and grid sweeps expect before a sweep (the L sweep
+// sentinel, as the flat sweeps expect before a sweep (the flat L sweep
 // itself resets the U sweeps' outputs row by row).
 inline int reset_set_sweep_buffers(SolveSet& ss)
 {

@@ -137,7 +137,11 @@ int pc_sweeps(mtlg_pc* P, const mtlg_vec* x, mtlg_vec* y)
     }
     // flat sweeps (no chunked plan, or chosen by sweep_kernel) need the flat entries
     const bool chunked = pl.ok;
-    if (!chunked) MTLG_TRY(ensure_flat(P));
+    if (!chunked) {
+        MTLG_TRY(ensure_flat(P));
+        if (P->tmp_used) MTLG_TRY(fill_sentinel(c, P->tmp.p, size_t(P->n) * 8));
+    }
+    P->tmp_used = chunked;
     MTLG_TRY(pc_views(P, sizeof(T) == 4 ? 1 : 0, d.L, d.U));
     MTLG_CUDA(cudaMemcpyAsync(P->desc.p, &d, sizeof d, cudaMemcpyHostToDevice, c->stream));
     if (chunked) {
@@ -145,7 +149,7 @@ int pc_sweeps(mtlg_pc* P, const mtlg_vec* x, mtlg_vec* y)
         memset(&op, 0, sizeof op);
         op.skip = SKIP_NONE;
         op.sleep_ns = c->sweep_sleep_ns;
-        // y0 = L^{-1} x  (temp, slot 0); clears y row by row
+        // y0 = L^{-1} x  (temp, slot 0); the chunked sweep clears y row by row
         op.tasks = pl.tl.p; op.ntasks = pl.ntl; op.ticket = P->tickets.p + 2; op.which = 0;
         op.in = SLOT_X; op.out = 0; op.reset = SLOT_B;
         MTLG_TRY((launch_chunk_sweep<T, S>(c, c->stream, sv, op, pl)));
