@@ -54,6 +54,7 @@ constexpr int kGridG = 8;                    // steps per staged block
 constexpr int kGridNB = 4;                   // staged blocks per warp (factor values and right-hand sides)
 constexpr int kGridRing = kGridG * kGridNB;  // rows of a ring (right-hand sides, results)
 constexpr int kGridH = 4;                    // steps between hand-offs inside a CTA
+constexpr int kGridTell = 5;                 // lanes that publish a step count (own, two readers, two writers)
 constexpr int kGridRecvWarps = 2;            // receiver warps: z sides, y sides
 constexpr int kGridDiagRows = 8192;          // rows per tile of a factor without entries
 static_assert(kGridStepPad % kGridG == 0, "layout padding must hold whole staged blocks");
@@ -190,20 +191,38 @@ __device__ __forceinline__ int grid_read(unsigned p)
 }
 // After reading a count: what its writer stored before is visible from here on.
 __device__ __forceinline__ void grid_acquire() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
-// Waits until both counts reach their needs (bounded: on expiry, or when
-// another wait has expired, the warp goes on with whatever the rings hold).
-__device__ __forceinline__ void grid_wait(unsigned p, int need, unsigned p2, int need2, int* err, long long lim)
+// Whether a warp's bounded wait ends without its value: after lim polls
+// (recorded as a timeout), or when another wait has expired.  Decided by all
+// lanes together, every lane having counted the same polls: the waits below
+// and what follows them use warp-wide votes.
+__device__ __forceinline__ bool grid_give_up(long long& spins, int* err, long long lim)
+{
+    const bool over = ++spins > (lim > 0 ? lim : kSpinLimit);
+    if (!over && (spins & 255) != 0) return false;
+    if (over) atomicExch(err, 1);
+    return __any_sync(0xffffffffu, over || *(volatile int*)err);
+}
+// Waits until the count reaches `need` (on expiry the warp goes on with
+// whatever the rings hold).
+__device__ __forceinline__ void grid_wait(unsigned p, int need, int* err, long long lim)
 {
     long long spins = 0;
-    while (__any_sync(0xffffffffu, grid_read(p) < need || grid_read(p2) < need2)) {
-        if ((++spins & 255) == 0 && *(volatile int*)err) break;
-        if (spins > (lim > 0 ? lim : kSpinLimit)) {
-            atomicExch(err, 1);
-            break;
-        }
-    }
+    while (__any_sync(0xffffffffu, grid_read(p) < need))
+        if (grid_give_up(spins, err, lim)) break;
     __syncwarp();
     grid_acquire();
+}
+// A compute warp's four counts, kept in one 16-byte slot that the other warps
+// write into: steps done by the writers of its y and z neighbours' rows and by
+// the readers of its own.
+struct GridCounts {
+    int y, z, yfree, zfree;
+};
+__device__ __forceinline__ GridCounts grid_counts(unsigned p)
+{
+    GridCounts c;
+    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(c.y), "=r"(c.z), "=r"(c.yfree), "=r"(c.zfree) : "r"(p) : "memory");
+    return c;
 }
 // A staged block's barrier (own copies: a fixed bound, given up early once a
 // wait has expired; the helper waits for every copy before the tile ends).
@@ -218,6 +237,19 @@ __device__ __forceinline__ void grid_bar_wait(unsigned long long* bar, unsigned 
         }
     }
 }
+// Whether the barrier's phase is over, without waiting.
+__device__ __forceinline__ bool mbar_test(unsigned long long* bar, unsigned parity)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // The thread's earlier cp.async copies arrive on the barrier when they land.
 __device__ __forceinline__ void cp_async_arrive(unsigned long long* bar)
 {
@@ -227,8 +259,8 @@ __device__ __forceinline__ void cp_async_arrive(unsigned long long* bar)
 // Shared-memory addresses of a tile's parts.
 struct GridSmem {
     unsigned stage, rings;            // factor blocks, rings (per warp: results, right-hand sides; then the receiver's)
-    unsigned prog, vy, vz, inf;       // step counts: compute warps, the receivers' y and z rows, never-waiting
-    unsigned zero;                    // a cell that holds +0
+    unsigned prog;                    // step counts of the compute warps (and a cell nobody reads)
+    unsigned slots;                   // GridCounts of the compute warps
     unsigned long long* full;         // the staged blocks' barriers, kGridNB per warp
     unsigned* blks;                   // staged blocks each warp has gone through before this tile
 };
@@ -237,11 +269,10 @@ struct GridSmem {
 template <typename T>
 struct GridWarp {
     unsigned stage, rhs, ring;        // staged factor blocks, right-hand-side ring, result ring
-    unsigned yin, zin;                // the y and z neighbours' columns (lanes at the warp's lower sides)
-    unsigned yp, zp;                  // bytes between their rows; no neighbour: 0, and yin / zin a cell that holds +0
-    unsigned yprog, zprog;            // step counts of those rings' writers
-    unsigned yfree, zfree;            // step counts of the own ring's readers
-    unsigned prog;                    // own step count
+    unsigned yin, zin;                // the y and z neighbours' columns (lanes at the warp's lower sides; no neighbour: a column of +0)
+    unsigned slot;                    // own GridCounts
+    int cy, cz, cyf, czf;             // what they have to exceed the next half's first step by (INT_MIN: nobody to wait for)
+    unsigned tell;                    // lanes below kGridTell: where the own step count goes
     unsigned long long* full;
     T* yhalo;                         // the lane's place in the hand-off row of step 0
     T* zhalo;
@@ -297,22 +328,37 @@ __device__ __forceinline__ void grid_compute(const GridWarp<T>& g)
             for (int k = 0; k < SL; ++k) lds(e + u * SB + k * (32 * unsigned(sizeof(S))), d.a[u][k]);
         }
     };
-    auto near = [&](GridHalf<T, S, SL>& d, int u, int s) {   // step u's neighbours' values (s: the half's first step)
-        lds(g.yin + unsigned((s + u + Sh::LY - 1) & (kGridRing - 1)) * g.yp, d.yv[u]);
+    // step u's neighbours' values in the half at step 8 m + h: ring row of that
+    // step + LY - 1 (LZ - 1), in block m, m + 1 or (LY 32) m + 3, m + 4
+    auto near = [&](GridHalf<T, S, SL>& d, int u, int h, unsigned r0, unsigned r1, unsigned r3, unsigned r4) {
+        constexpr int DY = (Sh::LY - 1) % G, BY = (Sh::LY - 1) / G, DZ = Sh::LZ - 1;
+        static_assert((BY == 0 || BY == 3) && DZ < G, "8 or 32 lines along y");
+        const int y = h + u + DY, z = h + u + DZ;
+        lds(g.yin + (y < G ? (BY ? r3 : r0) : (BY ? r4 : r1)) + (y % G) * P, d.yv[u]);
         d.zv[u] = T(0);
-        if (NS == 3) lds(g.zin + unsigned((s + u + Sh::LZ - 1) & (kGridRing - 1)) * g.zp, d.zv[u]);
+        if (NS == 3) lds(g.zin + (z < G ? r0 : r1) + (z % G) * P, d.zv[u]);
     };
-    auto wait_near = [&](int s) {   // the neighbours' values of the half at step s
-        grid_wait(g.yprog, min(s + H + Sh::LY - 1, total), g.zprog, min(s + H + Sh::LZ - 1, total), g.err, g.spin);
+    auto ready = [&](const GridCounts& c, int s) { return c.y - s >= g.cy && c.z - s >= g.cz; };   // for the half at step s
+    auto room = [&](const GridCounts& c, int s) { return c.yfree - s >= g.cyf && c.zfree - s >= g.czf; };   // for its results
+    auto wait_for = [&](auto test, int s) {
+        long long spins = 0;
+        while (__any_sync(0xffffffffu, !test(grid_counts(g.slot), s)))
+            if (grid_give_up(spins, g.err, g.spin)) break;
+        __syncwarp();
+        grid_acquire();
     };
+    auto ringrow = [&](int m) { return unsigned((m * G) & (kGridRing - 1)) * P; };
     // result of the last step, and the y and z lower lanes' (+0 before a lane's first row)
     T out = T(0), sy = T(0), sz = T(0);
     T* yh = g.yhalo;
     T* zh = g.zhalo;
-    auto half = [&](GridHalf<T, S, SL>& c, GridHalf<T, S, SL>& n, int m, int s0, unsigned enext, bool more) {
-        const int s1 = s0 + H;
-        const unsigned row = unsigned(s0 & (kGridRing - 1)) * P, rown = unsigned(s1 & (kGridRing - 1)) * P;
-        const int fy = grid_read(g.yprog), fz = grid_read(g.zprog), ry = grid_read(g.yfree), rz = grid_read(g.zfree);
+    // half h (0 or H) of block m from c's operands; the next half's into n
+    auto half = [&](GridHalf<T, S, SL>& c, GridHalf<T, S, SL>& n, int m, auto hc, unsigned enext, bool more) {
+        constexpr int h = decltype(hc)::value, hn = H - h;
+        const int s0 = m * G + h, s1 = s0 + H, mn = h == 0 ? m : m + 1;
+        const unsigned row = ringrow(m) + h * P, rown = ringrow(mn) + hn * P;
+        const unsigned r0 = ringrow(mn), r1 = ringrow(mn + 1), r3 = NS == 3 ? 0u : ringrow(mn + 3), r4 = r0;   // ring of four blocks
+        const GridCounts cnt = grid_counts(g.slot);
         T o[H];
 #pragma unroll
         for (int u = 0; u < H; ++u) {
@@ -362,17 +408,17 @@ __device__ __forceinline__ void grid_compute(const GridWarp<T>& g)
             // (after the last block: stale shared memory, never used)
             own(n, u, rown, enext);
             if (u == 0) grid_acquire();
-            if (u > 0) near(n, u - 1, s1);
-            if (u == H - 1) near(n, u, s1);
+            if (u > 0) near(n, u - 1, hn, r0, r1, r3, r4);
+            if (u == H - 1) near(n, u, hn, r0, r1, r3, r4);
         }
-        const bool ok = fy >= min(s1 + H + Sh::LY - 1, total) && fz >= min(s1 + H + Sh::LZ - 1, total);
+        // (voted: lanes may have read the counts at different times)
+        const bool ok = __all_sync(0xffffffffu, ready(cnt, s1) && room(cnt, s1));
         // the rows these results go to held those of a whole ring of steps ago
-        if (ry < s1 - kGridRing - (Sh::LY - 1) || rz < s1 - kGridRing - (Sh::LZ - 1))
-            grid_wait(g.yfree, s1 - kGridRing - (Sh::LY - 1), g.zfree, s1 - kGridRing - (Sh::LZ - 1), g.err, g.spin);
+        if (!ok) wait_for(room, s1);
 #pragma unroll
         for (int u = 0; u < H; ++u) sts(g.ring + row + u * P, o[u]);
         __syncwarp();
-        if (g.lane == 0) grid_count(g.prog, s1);
+        if (g.lane < kGridTell) grid_count(g.tell, s1 < total ? s1 : INT_MAX);
         if (g.yface) {
 #pragma unroll
             for (int u = 0; u < H; ++u) st_relaxed_gpu(yh + u * Sh::LZ, unsentinel(o[u]));
@@ -386,9 +432,9 @@ __device__ __forceinline__ void grid_compute(const GridWarp<T>& g)
             zh += H * Sh::LY;
         }
         if (more && !ok) {
-            wait_near(s1);
+            wait_for(ready, s1);
 #pragma unroll
-            for (int u = 0; u < H; ++u) near(n, u, s1);
+            for (int u = 0; u < H; ++u) near(n, u, hn, r0, r1, r3, r4);
         }
     };
     auto block = [&](int m) { return g.stage + ((g.blk + unsigned(m)) % kGridNB) * (G * SB); };
@@ -399,15 +445,16 @@ __device__ __forceinline__ void grid_compute(const GridWarp<T>& g)
     bar(0);
 #pragma unroll
     for (int u = 0; u < H; ++u) own(A, u, 0u, block(0));
-    wait_near(0);
+    wait_for(ready, 0);
 #pragma unroll
-    for (int u = 0; u < H; ++u) near(A, u, 0);
+    for (int u = 0; u < H; ++u) near(A, u, 0, ringrow(0), ringrow(1), NS == 3 ? 0u : ringrow(3), ringrow(0));
 #pragma unroll 1
     for (int m = 0; m < g.nblk; ++m) {
-        half(A, B, m, m * G, block(m) + H * SB, true);
-        const bool more = m + 1 < g.nblk;
-        if (more) bar(m + 1);
-        half(B, A, m, m * G + H, block(m + 1), more);
+        const unsigned q = g.blk + unsigned(m) + 1;
+        const bool more = m + 1 < g.nblk, landed = mbar_test(&g.full[q % kGridNB], (q / kGridNB) & 1u);
+        half(A, B, m, std::integral_constant<int, 0>(), block(m) + H * SB, true);
+        if (more && !landed) bar(m + 1);
+        half(B, A, m, std::integral_constant<int, H>(), block(m + 1), more);
     }
 }
 
@@ -416,7 +463,7 @@ __device__ __forceinline__ void grid_compute(const GridWarp<T>& g)
 // 8 m .. 8 m + 7, consecutive in x).
 template <typename T, typename S, int NW, int NS, bool REV, int OPK>
 __device__ __forceinline__ void grid_help(const S* src, unsigned stage, const T* vin, T* vout, unsigned rhs, unsigned ring,
-                                          unsigned prog, unsigned inf, unsigned long long* full, unsigned blk, int n, int nx,
+                                          unsigned prog, unsigned long long* full, unsigned blk, int n, int nx,
                                           int ny, int nz, int j0, int k0, int nblk, int lane, int* err, long long spin)
 {
     typedef GridShapeOf<NW, NS> Sh;
@@ -456,7 +503,7 @@ __device__ __forceinline__ void grid_help(const S* src, unsigned stage, const T*
     for (int m = 0; m < kGridNB && m < nblk; ++m) fetch(m);
 #pragma unroll 1
     for (int m = 0; m < nblk; ++m) {
-        grid_wait(prog, (m + 1) * G, inf, 0, err, spin);
+        grid_wait(prog, (m + 1) * G, err, spin);
         const unsigned cell = ring + (((m * G) & (kGridRing - 1)) + xo) * P + l0 * unsigned(sizeof(T));
         T v[8];
 #pragma unroll
@@ -484,11 +531,12 @@ __device__ __forceinline__ void grid_help(const S* src, unsigned stage, const T*
 // A receiver warp: polls the hand-off rows of up to NG warps of earlier
 // tiles (`src`: rows of WD elements, one per step), puts each complete prefix
 // of rows into its ring (columns col + WD g) with the sentinel back in its
-// place, and publishes the count of rows there.  A thread holds VN elements
+// place, and publishes the count of rows there (group g is read by compute
+// warp g * step: its count at `reader`, its slot's at `count`).  A thread holds VN elements
 // (16 bytes) of a row, so a group's poll is one coalesced load or a few.
 template <typename T, int WD, int NG>
 __device__ __forceinline__ void grid_receive(T* const (&src)[NG], int total, unsigned ring, int col, unsigned count,
-                                             unsigned reader, int reader_step, int slack, int lane, int* err, long long spin)
+                                             unsigned reader, int step, int slack, int lane, int* err, long long spin)
 {
     constexpr int VN = WD * int(sizeof(T)) >= 16 ? 16 / int(sizeof(T)) : 1;   // elements per thread
     constexpr int TR = WD / VN;                                              // threads per row
@@ -519,7 +567,7 @@ __device__ __forceinline__ void grid_receive(T* const (&src)[NG], int total, uns
 #pragma unroll
         for (int g = 0; g < NG; ++g) {
             if (!((left >> g) & 1u)) continue;
-            const int room = grid_read(reader + g * reader_step) + slack + kGridRing;   // rows below this are free
+            const int room = grid_read(reader + 4 * step * g) + slack + kGridRing;   // rows below this are free
             grid_acquire();
             int rows = 0;
             bool go = true;
@@ -545,21 +593,16 @@ __device__ __forceinline__ void grid_receive(T* const (&src)[NG], int total, uns
                 moved = true;
                 c[g] += rows;
                 __syncwarp();
-                if (lane == 0) grid_count(count + 4 * g, c[g]);
+                if (lane == 0) grid_count(count + 16 * step * g, c[g] < total ? c[g] : INT_MAX);
                 if (c[g] >= total) left &= ~(1u << g);
             }
         }
-        if (moved) continue;
-        if ((++spins & 255) == 0 && *(volatile int*)err) break;
-        if (spins > (spin > 0 ? spin : kSpinLimit)) {
-            if (lane == 0) atomicExch(err, 1);
-            break;
-        }
+        if (!moved && grid_give_up(spins, err, spin)) break;
     }
     __syncwarp();
     // after an expired wait nobody waits on these rows any more
     if (left && lane == 0)
-        for (int g = 0; g < NG; ++g) grid_count(count + 4 * g, INT_MAX);
+        for (int g = 0; g < NG; ++g) grid_count(count + 16 * step * g, INT_MAX);
 }
 
 // The roles of one tile's warps (NS and FAR from the factor).  Not inlined:
@@ -589,7 +632,7 @@ __device__ __noinline__ void grid_tile(const TriFactor& F, int n, const T* vin, 
                 const int ju = ty * Sh::WY + a;
                 src[a] = tz > 0 && ju < njb ? zh + (size_t(tz - 1) * njb + ju) * total * Sh::LY : nullptr;
             }
-            grid_receive<T, Sh::LY, Sh::WY>(src, total, rring, 0, sm.vz, sm.prog, 4, Sh::LZ - 1, lane, err, spin);
+            grid_receive<T, Sh::LY, Sh::WY>(src, total, rring, 0, sm.slots + 4, sm.prog, 1, Sh::LZ - 1, lane, err, spin);
         }
         return;
     }
@@ -600,7 +643,7 @@ __device__ __noinline__ void grid_tile(const TriFactor& F, int n, const T* vin, 
             const int ku = tz * Sh::WZ + a;
             src[a] = ty > 0 && ku < nkb ? yh + (size_t(ty - 1) * nkb + ku) * total * Sh::LZ : nullptr;
         }
-        grid_receive<T, Sh::LZ, Sh::WZ>(src, total, rring, Sh::ZCOLS, sm.vy, sm.prog, 4 * Sh::WY, Sh::LY - 1, lane, err, spin);
+        grid_receive<T, Sh::LZ, Sh::WZ>(src, total, rring, Sh::ZCOLS, sm.slots, sm.prog, Sh::WY, Sh::LY - 1, lane, err, spin);
         return;
     }
     const int w = warp % NW, wy = w % Sh::WY, wz = w / Sh::WY;
@@ -611,7 +654,7 @@ __device__ __noinline__ void grid_tile(const TriFactor& F, int n, const T* vin, 
     if (warp >= NW) {
         const S* src = static_cast<const S*>(F.gdata) + (size_t(ku) * njb + ju) * size_t(F.gnsp) * size_t(SL) * 32;
         grid_help<T, S, NW, NS, REV, OPK>(src, sm.stage + w * SE, vin, vout, ring + RB, ring, sm.prog + 4 * w,
-                                          sm.inf, sm.full + w * kGridNB, blk, n, nx, ny, nz, j0, k0, nblk, lane, err, spin);
+                                          sm.full + w * kGridNB, blk, n, nx, ny, nz, j0, k0, nblk, lane, err, spin);
         return;
     }
     const int ly = lane % Sh::LY, lz = lane / Sh::LY, j = j0 + ly, k = k0 + lz;
@@ -621,15 +664,24 @@ __device__ __noinline__ void grid_tile(const TriFactor& F, int n, const T* vin, 
     g.rhs = ring + RB + lane * TS;
     g.ring = ring + lane * TS;
     const bool has_y = ju > 0, has_z = NS == 3 && ku > 0;
-    g.yprog = !has_y ? sm.inf : wy > 0 ? sm.prog + 4 * (w - 1) : sm.vy + 4 * wz;
-    g.yin = !has_y ? sm.zero : wy > 0 ? ring - RW + (Sh::LY - 1 + Sh::LY * lz) * TS : rring + (Sh::ZCOLS + wz * Sh::LZ + lz) * TS;
-    g.zprog = !has_z ? sm.inf : wz > 0 ? sm.prog + 4 * (w - Sh::WY) : sm.vz + 4 * wy;
-    g.yp = has_y ? P : 0u;
-    g.zin = !has_z ? sm.zero : wz > 0 ? ring - Sh::WY * RW + (Sh::LY * (Sh::LZ - 1) + ly) * TS : rring + (wy * Sh::LY + ly) * TS;
-    g.zp = has_z ? P : 0u;
-    g.yfree = wy + 1 < Sh::WY && ju + 1 < njb ? sm.prog + 4 * (w + 1) : sm.inf;
-    g.zfree = wz + 1 < Sh::WZ && ku + 1 < nkb ? sm.prog + 4 * (w + Sh::WY) : sm.inf;
-    g.prog = sm.prog + 4 * w;
+    const unsigned zero = rring + 32 * TS;   // the receivers' ring keeps its first pad column +0
+    g.yin = !has_y ? zero : wy > 0 ? ring - RW + (Sh::LY - 1 + Sh::LY * lz) * TS : rring + (Sh::ZCOLS + wz * Sh::LZ + lz) * TS;
+    g.zin = !has_z ? zero : wz > 0 ? ring - Sh::WY * RW + (Sh::LY * (Sh::LZ - 1) + ly) * TS : rring + (wy * Sh::LY + ly) * TS;
+    // the half at step s reads its neighbours' rows of steps below s + kGridH
+    // + LY - 1 (LZ - 1); results of steps below s replace rows that readers
+    // have left once they are past s - kGridRing - (LY - 1)
+    const bool yr = wy + 1 < Sh::WY && ju + 1 < njb, zr = wz + 1 < Sh::WZ && ku + 1 < nkb;
+    g.slot = sm.slots + 16 * w;
+    g.cy = has_y ? kGridH + Sh::LY - 1 : INT_MIN;
+    g.cz = has_z ? kGridH + Sh::LZ - 1 : INT_MIN;
+    g.cyf = yr ? -kGridRing - (Sh::LY - 1) : INT_MIN;
+    g.czf = zr ? -kGridRing - (Sh::LZ - 1) : INT_MIN;
+    g.tell = lane == 0 ? sm.prog + 4 * w
+             : lane == 1 && yr ? sm.slots + 16 * (w + 1)
+             : lane == 2 && zr ? sm.slots + 16 * (w + Sh::WY) + 4
+             : lane == 3 && wy > 0 ? sm.slots + 16 * (w - 1) + 8
+             : lane == 4 && wz > 0 ? sm.slots + 16 * (w - Sh::WY) + 12
+                                   : sm.prog + 4 * NW;
     g.full = sm.full + w * kGridNB;
     g.lane_on = j < ny && k < nz;
     g.yface = wy == Sh::WY - 1 && ju + 1 < njb && ly == Sh::LY - 1;
@@ -660,18 +712,15 @@ __global__ void __launch_bounds__(32 * (2 * NW + kGridRecvWarps), 1) k_sweep_gri
     extern __shared__ __align__(128) unsigned char grid_smem[];
     __shared__ __align__(8) unsigned long long full[NW * kGridNB];
     __shared__ int s_task, s_go;
-    __shared__ int prog[2 * NW + 4];   // step counts: compute warps, the receivers' y rows, their z rows; never waited on
+    __shared__ int prog[NW + 1];
+    __shared__ __align__(16) int slots[4 * NW];
     __shared__ unsigned blks[NW];
-    __shared__ __align__(8) T zero;
     constexpr int SE = kGridRing * grid_cap(OPK) * 32;
     GridSmem sm;
     sm.stage = smem_u32(grid_smem);
     sm.rings = sm.stage + unsigned(NW * SE * int(sizeof(S)));
     sm.prog = smem_u32(prog);
-    sm.vy = sm.prog + 4 * NW;
-    sm.vz = sm.vy + 4 * (NW + 1);   // 2D tiles: one y row per tile; 3D: NW / 2 y rows, two z rows
-    sm.inf = sm.vz + 4 * 2;
-    sm.zero = smem_u32(&zero);
+    sm.slots = smem_u32(slots);
     sm.full = full;
     sm.blks = blks;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -681,7 +730,11 @@ __global__ void __launch_bounds__(32 * (2 * NW + kGridRecvWarps), 1) k_sweep_gri
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (tid < NW) blks[tid] = 0;
-    if (tid == 0) zero = T(0);
+    if (tid < kGridRing) {
+        // the pad column that stands for absent neighbours
+        const unsigned rw = (OPK == kGridSweep ? 2u : 1u) * unsigned(kGridRing * grid_pitch<T>() * int(sizeof(T)));
+        sts(sm.rings + NW * rw + unsigned(tid * grid_pitch<T>() + 32) * unsigned(sizeof(T)), T(0));
+    }
     __syncthreads();
     for (;;) {
         if (tid == 0) {
@@ -690,8 +743,8 @@ __global__ void __launch_bounds__(32 * (2 * NW + kGridRecvWarps), 1) k_sweep_gri
             s_task = t;
             s_go = t < op.ntasks && !skip_system(sv.st[op.tasks[t].sys], op.skip) && !*(volatile int*)sv.err;
         }
-        if (tid >= 32 && tid < 32 + 2 * NW + 3) prog[tid - 32] = 0;
-        if (tid == 32 + 2 * NW + 3) prog[tid - 32] = INT_MAX;
+        if (tid >= 32 && tid < 32 + 4 * NW) slots[tid - 32] = 0;
+        if (tid >= 64 && tid < 64 + NW) prog[tid - 64] = 0;
         __syncthreads();
         const int t = s_task;
         if (t >= op.ntasks) break;
