@@ -226,13 +226,14 @@ struct SetView {
     const int* sys_tile_begin;   // [n_sys + 1]
     SysDesc* desc;
     SysState* st;
-    double* partials;            // [n_tiles * kMaxDots]
+    double* partials;            // [kMaxDots][n_tiles]
     unsigned* counters;          // [n_sys] last-block counters (self-resetting)
     int* running;                // systems still running
     int* err;                    // device error flags (timeouts)
     unsigned long long cond;     // cudaGraphConditionalHandle (0: not in a graph)
     int use_cond;
     long long spin;              // polls before a dependency wait gives up (context "spin_limit"; 0: kSpinLimit)
+    int short_rows;              // every system's rows are short and regular (csr_short_rows): SpMV by thread per row
 };
 
 // ----------------------------------------------------------------- device helpers
@@ -318,7 +319,7 @@ __device__ __forceinline__ void store_partials(const SetView& sv, int tile, cons
 {
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int j = 0; j < ND; ++j) sv.partials[(long long)tile * kMaxDots + j] = v[j];
+        for (int j = 0; j < ND; ++j) sv.partials[(long long)j * sv.n_tiles + tile] = v[j];
     }
 }
 
@@ -357,31 +358,99 @@ __device__ __forceinline__ bool publish_tally(const SetView& sv, TileTally& tt)
 }
 
 // Sum of a system's tile partials (its first `count` tiles, or all of its
-// SpMV tiles) in tile order (deterministic: thread i adds tiles i,
-// i + blockDim, ... in turn, loads issued 8 tiles at a time); called by the
+// SpMV tiles) of ND dots in tile order (deterministic: thread i adds tiles i,
+// i + blockDim, ... in turn, loads issued 32 / ND tiles at a time: the one
+// CTA that does this is the tail of every reducing pass); called by the
 // whole last CTA, result valid in thread 0.
 template <int ND>
-__device__ __forceinline__ void gather_partials(const SetView& sv, int sys, double (&out)[ND], double* smem,
+__device__ __forceinline__ void gather_dots(const SetView& sv, int t0, int t1, double (&out)[kMaxDots], double* smem)
+{
+    constexpr int NU = 32 / ND;
+    const int B = blockDim.x;
+    double sum[ND];
+#pragma unroll
+    for (int j = 0; j < ND; ++j) sum[j] = 0.0;
+    for (int t = t0 + threadIdx.x; t < t1; t += NU * B) {
+        double v[NU][ND];
+#pragma unroll
+        for (int u = 0; u < NU; ++u)
+#pragma unroll
+            for (int j = 0; j < ND; ++j)
+                v[u][j] = t + u * B < t1 ? __ldcg(&sv.partials[(long long)j * sv.n_tiles + t + u * B]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < NU; ++u)
+#pragma unroll
+            for (int j = 0; j < ND; ++j)
+                if (t + u * B < t1) sum[j] += v[u][j];
+    }
+    block_reduce<ND>(sum, smem);
+#pragma unroll
+    for (int j = 0; j < kMaxDots; ++j) out[j] = 0.0;
+#pragma unroll
+    for (int j = 0; j < ND; ++j) out[j] = sum[j];
+}
+__device__ __forceinline__ void gather_partials(const SetView& sv, int sys, int nd, double (&out)[kMaxDots], double* smem,
                                                 int count = -1)
 {
     const int t0 = sv.sys_tile_begin[sys], t1 = count >= 0 ? t0 + count : sv.sys_tile_begin[sys + 1];
-    const int B = blockDim.x;
+    if (nd <= 1) gather_dots<1>(sv, t0, t1, out, smem);
+    else if (nd == 2) gather_dots<2>(sv, t0, t1, out, smem);
+    else gather_dots<kMaxDots>(sv, t0, t1, out, smem);
+}
+
+// Sums of NV values over the lanes of a warp, all at once (NV 1, 2, 4 or 8):
+// in the first log2(NV) steps lanes trade half of their values each, so a
+// step costs half the shuffles of the one before.  Every value is added over
+// the same pairs of lanes as a shuffle-down tree, so lane `l` with l % (32 /
+// NV) == 0 holds the tree's sum of value warp_sum_index<NV>(l), to the bit.
+template <int NV>
+__device__ __forceinline__ double warp_sums(double (&v)[NV])
+{
+    const int lane = threadIdx.x & 31;
+    int o = 16;
 #pragma unroll
-    for (int j = 0; j < ND; ++j) out[j] = 0.0;
-    for (int t = t0 + threadIdx.x; t < t1; t += 8 * B) {
-        double v[8][ND];
+    for (int half = NV / 2; half >= 1; half /= 2) {
+        const bool up = (lane & o) != 0;
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-#pragma unroll
-            for (int j = 0; j < ND; ++j)
-                v[u][j] = t + u * B < t1 ? __ldcg(&sv.partials[(long long)(t + u * B) * kMaxDots + j]) : 0.0;
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-#pragma unroll
-            for (int j = 0; j < ND; ++j)
-                if (t + u * B < t1) out[j] += v[u][j];
+        for (int k = 0; k < half; ++k) {
+            const double keep = up ? v[k + half] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, up ? v[k] : v[k + half], o);
+        }
+        o /= 2;
     }
-    block_reduce<ND>(out, smem);
+#pragma unroll
+    for (; o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+template <int NV>
+__device__ __forceinline__ int warp_sum_index(int lane)
+{
+    int idx = 0;
+#pragma unroll
+    for (int half = NV / 2, o = 16; half >= 1; half /= 2, o /= 2) idx += (lane & o) ? half : 0;
+    return idx;
+}
+
+// Per-warp partial dots of up to kPartTiles tiles wait in shared memory
+// ([tile][warp][dot]) until one pass adds each tile's warps, in the order
+// block_reduce adds them, and stores the tiles' partials: one barrier pair
+// per kPartTiles tiles instead of two per tile.
+constexpr int kPartTiles = 32;
+template <int ND>
+__device__ __forceinline__ void flush_parts(const SetView& sv, int tile, int count, const double* s_part)
+{
+    constexpr int NWP = kBlock / 32;
+    static_assert(NWP == 8, "the tree below adds eight warps");
+    __syncthreads();
+    for (int k = threadIdx.x; k < count * ND; k += kBlock) {
+        const double* w = s_part + k / ND * (NWP * ND) + k % ND;
+        double t[NWP];
+#pragma unroll
+        for (int q = 0; q < NWP; ++q) t[q] = w[q * ND] + 0.0;   // block_reduce adds the idle lanes' zeros
+        sv.partials[(long long)(k % ND) * sv.n_tiles + tile + k / ND] =
+            ((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7]));
+    }
+    __syncthreads();
 }
 
 // Phases of a served solve (continuous batching): each engine step runs the

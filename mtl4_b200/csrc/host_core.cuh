@@ -388,6 +388,15 @@ struct mtlg_csr {
 
 namespace mtlg {
 
+// Short, regular rows: at most kShortRow entries each and kScalarMeanRow on
+// average.  A thread per row then wins over staged tiles (128^3 7-point
+// product 45 us against 106 us), whose barriers and buffers pay off on
+// longer or uneven rows, where a thread's walk is uncoalesced.
+inline bool csr_short_rows(const mtlg_csr* A)
+{
+    return !A->irregular && A->n_rows > 0 && A->nnz <= int64_t(kScalarMeanRow) * A->n_rows;
+}
+
 inline int ensure_f32_values(mtlg_csr* A)
 {
     if (A->v32.p) return MTLG_OK;
@@ -431,6 +440,7 @@ inline int csr_op_set(mtlg_csr* A, SetView& sv)
     sv.err = A->misc.p + 1;
     sv.cond = 0;
     sv.use_cond = 0;
+    sv.short_rows = csr_short_rows(A) ? 1 : 0;
     return MTLG_OK;
 }
 
@@ -480,6 +490,26 @@ struct SpmvShape {
     }
 };
 template <typename T, int XF, int ASG> int SpmvShape<T, XF, ASG>::occ = 0;
+// k_spmv_short: CTAs per SM by number of dots.
+template <typename T, int XF, int ASG>
+struct ShortShape {
+    static int occ[3];
+    template <int ND>
+    static int query()
+    {
+        int o = 1;
+        MTLG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_spmv_short<T, XF, ASG, ND>, kBlock, 0));
+        occ[ND] = std::max(1, o);
+        return MTLG_OK;
+    }
+    static int init()
+    {
+        MTLG_TRY(query<0>());
+        MTLG_TRY(query<1>());
+        return query<2>();
+    }
+};
+template <typename T, int XF, int ASG> int ShortShape<T, XF, ASG>::occ[3] = {0, 0, 0};
 
 #define MTLG_SPMV_VARIANTS(M)      \
     M(XF_PLAIN, ASG_SET)          \
@@ -496,7 +526,9 @@ inline int init_kernel_shapes()
 {
 #define MTLG_SPMV_INIT(XF, ASG)                              \
     MTLG_TRY((SpmvShape<double, XF, ASG>::init()));          \
-    MTLG_TRY((SpmvShape<float, XF, ASG>::init()));
+    MTLG_TRY((SpmvShape<float, XF, ASG>::init()));           \
+    MTLG_TRY((ShortShape<double, XF, ASG>::init()));         \
+    MTLG_TRY((ShortShape<float, XF, ASG>::init()));
     MTLG_SPMV_VARIANTS(MTLG_SPMV_INIT)
 #undef MTLG_SPMV_INIT
     MTLG_CUDA(cudaFuncSetAttribute(k_dot_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDots * kRefWarpSmem));
@@ -561,6 +593,22 @@ inline int launch_spmv(mtlg_ctx* c, cudaStream_t st, const SetView& sv, const Sp
         MTLG_TRY(launch_spmv<T>(c, st, sv, plain, xf, asg));
         return launch_dot_ref(c, st, sv, r);
     }
+    if (sv.short_rows && op.ndot <= 2) {
+#define MTLG_SHORT_ND(XF, ASG, ND) k_spmv_short<T, XF, ASG, ND><<<grid, kBlock, 0, st>>>(sv, op)
+#define MTLG_SHORT_CASE(XF, ASG)                                                                  \
+    if (xf == XF && asg == ASG) {                                                                 \
+        const int nd = op.fin != FIN_NONE ? op.ndot : 0;                                          \
+        const int grid = std::min(sv.n_tiles, c->sm_count * ShortShape<T, XF, ASG>::occ[nd]);     \
+        if (nd == 0) MTLG_SHORT_ND(XF, ASG, 0);                                                   \
+        else if (nd == 1) MTLG_SHORT_ND(XF, ASG, 1);                                              \
+        else MTLG_SHORT_ND(XF, ASG, 2);                                                           \
+        c->launches++;                                                                            \
+        return MTLG_OK;                                                                           \
+    }
+        MTLG_SPMV_VARIANTS(MTLG_SHORT_CASE)
+#undef MTLG_SHORT_CASE
+#undef MTLG_SHORT_ND
+    }
     const int smem = 2 * StageLayout<T>::BYTES;
 #define MTLG_SPMV_CASE(XF, ASG)                                                                    \
     if (xf == XF && asg == ASG) {                                                                 \
@@ -590,9 +638,17 @@ inline int launch_vec(mtlg_ctx* c, cudaStream_t st, const SetView& sv, const Vec
     // one CTA per run of tiles, vec_ctas_per_sm per SM at most (each CTA
     // publishes its dot tally with one atomic on the system's counter)
     dim3 g(std::min(sv.n_tiles, c->vec_ctas_per_sm * c->sm_count)), b(kBlock);
+    if (op.ndot > 2) {
+        set_error("a vector pass reduces at most two dots");
+        return MTLG_ERR_NOT_SUPPORTED;
+    }
     switch (op.op) {
-#define MTLG_VEC_CASE(OP) \
-    case OP: k_vec<T, OP><<<g, b, 0, st>>>(sv, op); break;
+#define MTLG_VEC_CASE(OP)                                          \
+    case OP:                                                       \
+        if (op.ndot == 0) k_vec<T, OP, 0><<<g, b, 0, st>>>(sv, op);      \
+        else if (op.ndot == 1) k_vec<T, OP, 1><<<g, b, 0, st>>>(sv, op); \
+        else k_vec<T, OP, 2><<<g, b, 0, st>>>(sv, op);                   \
+        break;
         MTLG_VEC_CASE(VOP_DOT)
         MTLG_VEC_CASE(VOP_AXPY)
         MTLG_VEC_CASE(VOP_CG_UPDATE)

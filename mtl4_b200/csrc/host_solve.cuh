@@ -34,6 +34,7 @@ struct SolveSet {
     DBuf<SysDesc> desc, desc64;
     DBuf<SysState> st;
     int n_tiles = 0;
+    int short_rows = 0;   // every system's rows are short and regular
     DBuf<Tile> tiles;
     DBuf<int> stb;
     DBuf<double> partials;
@@ -87,6 +88,7 @@ struct SolveSet {
         v.cond = in_graph ? cond : 0;
         v.use_cond = in_graph ? 1 : 0;
         v.spin = ctx ? ctx->spin_limit : 0;
+        v.short_rows = short_rows;
         return v;
     }
 };
@@ -120,8 +122,10 @@ inline int build_set(mtlg_ctx* c, SolveSet& ss)
     std::vector<int> stb(ss.S + 1, 0);
     long long maxn = 1;
     bool all_identity = true, all_jacobi = true;
+    ss.short_rows = 1;
     for (int s = 0; s < ss.S; ++s) {
         const SysInput& si = ss.in[s];
+        if (si.A->n_rows > 0 && !csr_short_rows(si.A)) ss.short_rows = 0;
         plan_tiles(si.A->h_rp.data(), int(si.A->n_rows), s, tiles);
         stb[s + 1] = int(tiles.size());
         maxn = std::max<long long>(maxn, si.A->n_rows);

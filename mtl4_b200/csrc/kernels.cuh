@@ -324,6 +324,36 @@ struct RowEpilogue {
     }
 };
 
+template <typename T, int ASG, int XF>
+__device__ __forceinline__ RowEpilogue<T, ASG, XF> row_epilogue(const SysDesc& d, const SpmvOp& op)
+{
+    RowEpilogue<T, ASG, XF> epi;
+    epi.y = vptr<T>(d, op.y);
+    epi.y2 = op.y2 != SLOT_NONE ? vptr<T>(d, op.y2) : nullptr;
+    epi.w = op.w != SLOT_NONE ? vptr<T>(d, op.w) : nullptr;
+    epi.pnew = op.pnew != SLOT_NONE ? vptr<T>(d, op.pnew) : nullptr;
+    epi.ndot = op.ndot;
+    epi.a0 = {op.da[0], names_vector(op.da[0]) ? vptr<T>(d, op.da[0]) : nullptr};
+    epi.b0 = {op.db[0], names_vector(op.db[0]) ? vptr<T>(d, op.db[0]) : nullptr};
+    epi.c0 = {op.dc[0], names_vector(op.dc[0]) ? vptr<T>(d, op.dc[0]) : nullptr};
+    epi.a1 = {op.da[1], names_vector(op.da[1]) ? vptr<T>(d, op.da[1]) : nullptr};
+    epi.b1 = {op.db[1], names_vector(op.db[1]) ? vptr<T>(d, op.db[1]) : nullptr};
+    epi.c1 = {op.dc[1], names_vector(op.dc[1]) ? vptr<T>(d, op.dc[1]) : nullptr};
+    return epi;
+}
+template <typename T, int XF>
+__device__ __forceinline__ XIn<T, XF> row_input(const SysDesc& d, const SysState& s, const SpmvOp& op)
+{
+    XIn<T, XF> xin;
+    xin.x = vptr<T>(d, op.x);
+    xin.p = op.p != SLOT_NONE ? vptr<T>(d, op.p) : nullptr;
+    xin.z = op.z != SLOT_NONE ? vptr<T>(d, op.z) : nullptr;
+    xin.dinv = static_cast<const T*>(d.inv_diag);
+    xin.beta = T(s.beta);
+    xin.first = (s.iter == 0);
+    return xin;
+}
+
 // ---- shared-memory staging of a stream tile (16-byte cp.async copies)
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
 {
@@ -377,7 +407,7 @@ __device__ __forceinline__ void spmv_publish(const SetView& sv, const OpT& op, T
 {
     if (publish_tally(sv, tally)) {
         double tot[kMaxDots];
-        gather_partials<kMaxDots>(sv, tally.sys, tot, s_red);
+        gather_partials(sv, tally.sys, op.ndot, tot, s_red);
         if (threadIdx.x == 0) finalize(sv, op.fin, tally.sys, tot);
     }
 }
@@ -434,27 +464,10 @@ __global__ void __launch_bounds__(kBlock, 3) k_spmv(SetView sv, SpmvOp op)
         const SysDesc& d = sv.desc[sys];
         const SysState& s = sv.st[sys];
         if (!skip_system(s, op.skip)) {
-            XIn<T, XF> xin;
-            xin.x = vptr<T>(d, op.x);
-            xin.p = op.p != SLOT_NONE ? vptr<T>(d, op.p) : nullptr;
-            xin.z = op.z != SLOT_NONE ? vptr<T>(d, op.z) : nullptr;
-            xin.dinv = static_cast<const T*>(d.inv_diag);
-            xin.beta = T(s.beta);
-            xin.first = (s.iter == 0);
+            const XIn<T, XF> xin = row_input<T, XF>(d, s, op);
             const T* dinv = xin.dinv;
 
-            RowEpilogue<T, ASG, XF> epi;
-            epi.y = vptr<T>(d, op.y);
-            epi.y2 = op.y2 != SLOT_NONE ? vptr<T>(d, op.y2) : nullptr;
-            epi.w = op.w != SLOT_NONE ? vptr<T>(d, op.w) : nullptr;
-            epi.pnew = op.pnew != SLOT_NONE ? vptr<T>(d, op.pnew) : nullptr;
-            epi.ndot = op.ndot;
-            epi.a0 = {op.da[0], names_vector(op.da[0]) ? vptr<T>(d, op.da[0]) : nullptr};
-            epi.b0 = {op.db[0], names_vector(op.db[0]) ? vptr<T>(d, op.db[0]) : nullptr};
-            epi.c0 = {op.dc[0], names_vector(op.dc[0]) ? vptr<T>(d, op.dc[0]) : nullptr};
-            epi.a1 = {op.da[1], names_vector(op.da[1]) ? vptr<T>(d, op.da[1]) : nullptr};
-            epi.b1 = {op.db[1], names_vector(op.db[1]) ? vptr<T>(d, op.db[1]) : nullptr};
-            epi.c1 = {op.dc[1], names_vector(op.dc[1]) ? vptr<T>(d, op.dc[1]) : nullptr};
+            const RowEpilogue<T, ASG, XF> epi = row_epilogue<T, ASG, XF>(d, op);
             double d0 = 0.0, d1 = 0.0;
 
             if (tile.kind == TILE_STREAM) {
@@ -552,6 +565,108 @@ __global__ void __launch_bounds__(kBlock, 3) k_spmv(SetView sv, SpmvOp op)
         nxt = nn;
     }
     cp_async_wait_0();
+    if (op.fin != FIN_NONE) spmv_publish(sv, op, tally, s_red);
+}
+
+// ---------------------------------------------------------------- SpMV, thread per row
+// The in-solve product of sets whose rows are all short and regular
+// (SetView::short_rows): a thread takes one row of each tile straight from
+// global memory, entries 8 at a time in storage order (k_spmv's arithmetic to
+// the bit).  Bound by HBM: adjacent rows of a warp use the sectors the first
+// of them brought in, and there is no staging and no barrier per tile (FP64 BiCGSTAB product with two
+// dots on 128^3, cold caches: k_spmv 106 us, this kernel 80 us; floor 38 us at
+// 6.65 TB/s).
+// Each CTA walks a contiguous run of tiles.
+template <typename T, int XF, int ASG, int ND>
+__global__ void __launch_bounds__(kBlock, 2) k_spmv_short(SetView sv, SpmvOp op)
+{
+    __shared__ double s_red[kMaxDots * 32];
+    __shared__ double s_part[kPartTiles * (kBlock / 32) * (ND > 0 ? ND : 1)];
+    if (op.count_body && blockIdx.x == 0 && threadIdx.x == 0) {
+        int runs = atomicAdd(&sv.err[1], 1) + 1;   // bounds a graph while-loop (see k_spmv)
+        if (runs > sv.err[2] || *(volatile int*)sv.running <= 0) set_cond(sv, 0u);
+    }
+    const int t_begin = int((long long)sv.n_tiles * blockIdx.x / gridDim.x);
+    const int t_end = int((long long)sv.n_tiles * (blockIdx.x + 1) / gridDim.x);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    TileTally tally;
+    int t = t_begin;
+    while (t < t_end) {
+        const int sys = sv.n_sys == 1 ? 0 : sv.tiles[t].sys;
+        const int te = sv.n_sys == 1 ? t_end : min(t_end, sv.sys_tile_begin[sys + 1]);   // this system's tiles in the CTA's run
+        if (op.fin != FIN_NONE && sys != tally.sys) {
+            spmv_publish(sv, op, tally, s_red);
+            tally.sys = sys;
+        }
+        const SysState& s = sv.st[sys];
+        if (skip_system(s, op.skip)) {
+            t = te;
+            continue;
+        }
+        const SysDesc& d = sv.desc[sys];
+        const int* __restrict__ rp = d.rp;
+        const int* __restrict__ ci = d.ci;
+        const T* __restrict__ va = static_cast<const T*>(d.val);
+        const XIn<T, XF> xin = row_input<T, XF>(d, s, op);
+        const RowEpilogue<T, ASG, XF> epi = row_epilogue<T, ASG, XF>(d, op);
+        // Row bounds two tiles ahead, the first 8 columns one tile ahead: a
+        // tile then costs one round of loads (values and gathers), not the
+        // chain row pointers -> columns -> gathers.
+        auto tile_row = [&](int k) {   // this thread's row of tile k, or -1
+            const int r = sv.tiles[k].row_begin + int(threadIdx.x);
+            return k < te && r < sv.tiles[k].row_end ? r : -1;
+        };
+        auto bounds = [&](int r) { return r >= 0 ? make_int2(rp[r], rp[r + 1]) : make_int2(0, 0); };
+        int i = tile_row(t), in = t + 1 < te ? tile_row(t + 1) : -1;
+        int2 ae = bounds(i), aen = bounds(in);
+        int c[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) c[u] = ae.x + u < ae.y ? ci[ae.x + u] : 0;
+        int held = 0;
+        for (; t < te; ++t) {
+            const int a = ae.x, e = ae.y, q = fused_tail(a, e);
+            T xv[8], av[8], acc = T(0);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) if (a + u < e) { av[u] = va[a + u]; xv[u] = xin(c[u]); }
+            const int inn = t + 2 < te ? tile_row(t + 2) : -1;
+            const int2 aenn = bounds(inn);
+            int cn[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) cn[u] = aen.x + u < aen.y ? ci[aen.x + u] : 0;
+            double d0 = 0.0, d1 = 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) if (a + u < e) acc = row_step(acc, av[u], xv[u], a + u >= q);
+            for (int k = a + 8; k < e; k += 8) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) if (k + u < e) { av[u] = va[k + u]; xv[u] = xin(ci[k + u]); }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) if (k + u < e) acc = row_step(acc, av[u], xv[u], k + u >= q);
+            }
+            if (i >= 0) epi(i, acc, xin(i), xin.dinv, d0, d1);
+            i = in;
+            in = inn;
+            ae = aen;
+            aen = aenn;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) c[u] = cn[u];
+            if constexpr (ND > 0) {
+                double dd[ND];
+                dd[0] = d0;
+                if (ND > 1) dd[ND - 1] = d1;
+                const double sum = warp_sums<ND>(dd);
+                if (lane % (32 / ND) == 0) s_part[(held * (kBlock / 32) + warp) * ND + warp_sum_index<ND>(lane)] = sum;
+                if (++held == kPartTiles) {
+                    flush_parts<ND>(sv, t + 1 - held, held, s_part);
+                    tally.n += unsigned(held);
+                    held = 0;
+                }
+            }
+        }
+        if constexpr (ND > 0) {
+            if (held) flush_parts<ND>(sv, t - held, held, s_part);
+            tally.n += unsigned(held);
+        }
+    }
     if (op.fin != FIN_NONE) spmv_publish(sv, op, tally, s_red);
 }
 
@@ -797,12 +912,21 @@ struct VecOp {
     double scalar;
 };
 
-template <typename T>
-__device__ __forceinline__ T vpick(const T* const* v, int j, int code, int i, const T* dinv)
+// The vectors a pass writes, as dot factors see them: op.a (what is computed
+// first), and a second result (CG's and BiCGSTAB's r; the copies of the inner
+// right-hand side).
+template <int OP>
+__device__ __forceinline__ int vec_out1(const VecOp& op)
 {
-    if (code == OPND_ONE) return T(1);
-    if (code == OPND_D) return dinv[i];
-    return v[j][i];
+    return OP == VOP_AXPY || OP == VOP_CG_UPDATE || OP == VOP_BI_P || OP == VOP_BI_S || OP == VOP_BI_XR ? op.a : SLOT_NONE;
+}
+template <int OP>
+__device__ __forceinline__ bool vec_is_out2(const VecOp& op, int code)
+{
+    if (OP == VOP_CG_UPDATE) return code == op.c;
+    if (OP == VOP_BI_XR) return code == op.g;
+    if (OP == VOP_REF_CAST) return code == op.a || code == op.c || code == op.e;
+    return false;
 }
 
 // Publishes a CTA's tally of a system's finished vector-pass tiles; the CTA
@@ -814,7 +938,7 @@ __device__ __forceinline__ void vec_publish(const SetView& sv, const VecOp& op, 
     const int count = int(tally.need);
     if (publish_tally(sv, tally)) {
         double tot[kMaxDots];
-        gather_partials<kMaxDots>(sv, tally.sys, tot, s_red, count);
+        gather_partials(sv, tally.sys, op.ndot, tot, s_red, count);
         if (threadIdx.x == 0) {
             SysState& s = sv.st[tally.sys];
             if (OP == VOP_BI_XR && (s.flags & FLAG_FINISHING)) {
@@ -837,14 +961,20 @@ constexpr int kVecGroup = 4;   // tiles a vector-pass CTA works on at once (one 
 // kVecGroup tiles of one system at a time (thread k takes row k of each, so
 // its loads of the group's rows are in flight together, with no tile
 // metadata to read); the system's vectors and scalars are read once per run.
-// Each tile's partial dots are block reduced on their own in a fixed order,
-// so the sums do not depend on the grid, the grouping or the batch.
-template <typename T, int OP>
-__global__ void __launch_bounds__(kBlock) k_vec(SetView sv, VecOp op)
+// Each tile's partial dots are summed on their own in a fixed order, so the
+// sums do not depend on the grid, the grouping or the batch.  ND (0, 1 or 2):
+// the pass's dots; a group's are reduced together (warp_sums), and the warps'
+// sums meet in shared memory only every kPartTiles tiles, so the streams of
+// loads run on (FP64 BiCGSTAB x / r pass on 128^3: 84 us with a block
+// reduction of 16 values per group, 57 us so; floor 20 us at 6.65 TB/s).
+template <typename T, int OP, int ND>
+__global__ void __launch_bounds__(kBlock, 2) k_vec(SetView sv, VecOp op)
 {
     static_assert(kBlock == kTileRows, "a vector-pass thread takes one row of each tile");
-    constexpr int NR = kVecGroup * kMaxDots;
-    __shared__ double s_red[NR * 32];
+    static_assert(kPartTiles % kVecGroup == 0, "whole groups of tiles wait in shared memory");
+    constexpr int NV = ND > 0 ? ND : 1, NR = kVecGroup * NV;
+    __shared__ double s_red[kMaxDots * 32];
+    __shared__ double s_part[kPartTiles * (kBlock / 32) * NV];
     if (op.count_body && blockIdx.x == 0 && threadIdx.x == 0) {
         int runs = atomicAdd(&sv.err[1], 1) + 1;
         if (runs > sv.err[2] || *(volatile int*)sv.running <= 0) set_cond(sv, 0u);
@@ -854,11 +984,13 @@ __global__ void __launch_bounds__(kBlock) k_vec(SetView sv, VecOp op)
     TileTally tally;
     int t = t_begin;
     while (t < t_end) {
-        const int sys = sv.tiles[t].sys;
-        const int tb = sv.sys_tile_begin[sys];
-        const int te = min(t_end, sv.sys_tile_begin[sys + 1]);   // this system's tile indices in the CTA's range
+        // (a set of one system needs no look at the tiles)
+        const bool one = sv.n_sys == 1;
+        const int sys = one ? 0 : sv.tiles[t].sys;
+        const int tb = one ? 0 : sv.sys_tile_begin[sys];
+        const int te = one ? t_end : min(t_end, sv.sys_tile_begin[sys + 1]);   // this system's tile indices in the CTA's range
         const SysDesc& d = sv.desc[sys];
-        const int n = sv.tiles[sv.sys_tile_begin[sys + 1] - 1].row_end;   // its rows (the last tile's end)
+        const int n = d.n;   // its rows
         const int nvt = (n + kTileRows - 1) / kTileRows;                   // its row tiles
         if (sys != tally.sys) {
             vec_publish<OP>(sv, op, tally, s_red);
@@ -871,12 +1003,21 @@ __global__ void __launch_bounds__(kBlock) k_vec(SetView sv, VecOp op)
             continue;
         }
         const T* dinv = static_cast<const T*>(d.inv_diag);
-        const T* dv[3 * kMaxDots];
+        // Dot factors: a vector in memory, or a result of this pass (taken
+        // from the register it was just computed in: 1 what A gets, 2 the
+        // second result).
+        const T* dm[2 * NV];
+        int from[2 * NV];
+        bool by_d[NV];
 #pragma unroll
-        for (int j = 0; j < kMaxDots; ++j) {
-            dv[3 * j + 0] = (j < op.ndot && names_vector(op.da[j])) ? vptr<T>(d, op.da[j]) : nullptr;
-            dv[3 * j + 1] = (j < op.ndot && names_vector(op.db[j])) ? vptr<T>(d, op.db[j]) : nullptr;
-            dv[3 * j + 2] = (j < op.ndot && names_vector(op.dc[j])) ? vptr<T>(d, op.dc[j]) : nullptr;
+        for (int j = 0; j < ND; ++j) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int code = k == 0 ? op.da[j] : op.db[j];
+                from[2 * j + k] = code == vec_out1<OP>(op) ? 1 : vec_is_out2<OP>(op, code) ? 2 : 0;
+                dm[2 * j + k] = from[2 * j + k] == 0 && names_vector(code) ? vptr<T>(d, code) : nullptr;
+            }
+            by_d[j] = op.dc[j] == OPND_D;
         }
         T* A = op.a != SLOT_NONE ? vptr<T>(d, op.a) : nullptr;
         T* B = op.b != SLOT_NONE ? vptr<T>(d, op.b) : nullptr;
@@ -889,72 +1030,104 @@ __global__ void __launch_bounds__(kBlock) k_vec(SetView sv, VecOp op)
         const bool first = (s.iter <= 1);
         const double scale = s.scale;
         const bool reduce = op.fin != FIN_NONE || (OP == VOP_BI_XR && finishing);
-        // one row: the pass and its dot terms
-        auto row = [&](int i, double* dot) {
-            if (OP == VOP_AXPY) {
-                A[i] = fma(T(op.scalar), B[i], A[i]);                       // A += s B
-            } else if (OP == VOP_CG_UPDATE) {
-                A[i] = fma(alpha, B[i], A[i]);                              // x += alpha p
-                C[i] = fma(-alpha, E[i], C[i]);                             // r -= alpha q
-            } else if (OP == VOP_BI_P) {
-                // p = r + beta * (p - omega * v)     (bicgstab.hpp:49-53)
-                A[i] = first ? B[i] : fma(beta, fma(-omega, C[i], A[i]), B[i]);
-            } else if (OP == VOP_BI_S) {
-                A[i] = fma(-alpha, C[i], B[i]);                             // s = r - alpha v
-            } else if (OP == VOP_BI_XR) {
-                // A x, B phat, C shat, E s, F t, G r
-                if (finishing) {
-                    A[i] = fma(alpha, B[i], A[i]);                          // x += alpha phat
-                } else {
-                    // x += omega shat + alpha phat, evaluated as the reference
-                    // build does: x + fma(alpha, phat, omega shat)
-                    A[i] = A[i] + fma(alpha, B[i], omega * C[i]);
-                    G[i] = fma(-omega, F[i], E[i]);                         // r = s - omega t
-                }
-            } else if (OP == VOP_REF_CAST) {
-                // inner right-hand side float(r64 / ||r64||); inner x = 0, r = b
-                const T bi = T(d.r64[i] / scale);
-                A[i] = bi;
-                if (B) B[i] = T(0);
-                if (C) C[i] = bi;
-                if (E) E[i] = bi;
-            } else if (OP == VOP_REF_UPDATE) {
-                d.x64[i] = fma(scale, double(A[i]), d.x64[i]);            // x += ||r|| * d
-            } else if (OP == VOP_FILL) {
-                A[i] = T(op.scalar);
-            } else if (OP == VOP_COPY) {
-                A[i] = B[i];
-            } else if (OP == VOP_SCALE_COPY) {
-                A[i] = T(op.scalar) * B[i];
-            }
-#pragma unroll
-            for (int j = 0; j < kMaxDots; ++j)
-                if (j < op.ndot)
-                    dot[j] += double(vpick<T>(dv, 3 * j + 0, op.da[j], i, dinv) * vpick<T>(dv, 3 * j + 1, op.db[j], i, dinv) *
-                                     vpick<T>(dv, 3 * j + 2, op.dc[j], i, dinv));
-        };
+        int held = 0;   // tiles whose warp sums wait in shared memory
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         for (; t < te; t += kVecGroup) {
             const int v0 = t - tb;
             const int ng = max(0, min(min(kVecGroup, te - t), nvt - v0));   // row tiles among these indices
             double dot[NR];
 #pragma unroll
             for (int k = 0; k < NR; ++k) dot[k] = 0.0;
+            // all rows' loads, then their arithmetic and stores (a store
+            // between them would hold the next row's loads back)
+            T a[kVecGroup], b[kVecGroup], c[kVecGroup], e[kVecGroup], f[kVecGroup], dd[kVecGroup], m[kVecGroup][2 * NV];
+            double w[kVecGroup];
+            const int i0 = v0 * kTileRows + int(threadIdx.x);
 #pragma unroll
             for (int q = 0; q < kVecGroup; ++q) {
-                const int i = (v0 + q) * kTileRows + int(threadIdx.x);
-                if (q < ng && i < n) row(i, dot + q * kMaxDots);
+                const int i = i0 + q * kTileRows;
+                if (q >= ng || i >= n) continue;
+                if (OP == VOP_AXPY || OP == VOP_CG_UPDATE || OP == VOP_BI_XR || (OP == VOP_BI_P && !first) || OP == VOP_REF_UPDATE) a[q] = A[i];
+                if (OP == VOP_AXPY || OP == VOP_CG_UPDATE || OP == VOP_BI_P || OP == VOP_BI_S || OP == VOP_BI_XR || OP == VOP_COPY || OP == VOP_SCALE_COPY) b[q] = B[i];
+                if (OP == VOP_CG_UPDATE || (OP == VOP_BI_P && !first) || OP == VOP_BI_S || (OP == VOP_BI_XR && !finishing)) c[q] = C[i];
+                if (OP == VOP_CG_UPDATE || (OP == VOP_BI_XR && !finishing)) e[q] = E[i];
+                if (OP == VOP_BI_XR && !finishing) f[q] = F[i];
+                if (OP == VOP_REF_CAST) w[q] = d.r64[i];
+                if (OP == VOP_REF_UPDATE) w[q] = d.x64[i];
+#pragma unroll
+                for (int j = 0; j < 2 * ND; ++j) if (from[j] == 0) m[q][j] = dm[j] ? dm[j][i] : T(1);
+#pragma unroll
+                for (int j = 0; j < ND; ++j) if (by_d[j]) dd[q] = dinv[i];
+            }
+#pragma unroll
+            for (int q = 0; q < kVecGroup; ++q) {
+                const int i = i0 + q * kTileRows;
+                if (q >= ng || i >= n) continue;
+                T o1 = T(0), o2 = T(0);
+                if (OP == VOP_AXPY) {
+                    o1 = fma(T(op.scalar), b[q], a[q]);                     // A += s B
+                    A[i] = o1;
+                } else if (OP == VOP_CG_UPDATE) {
+                    o1 = fma(alpha, b[q], a[q]);                            // x += alpha p
+                    o2 = fma(-alpha, e[q], c[q]);                           // r -= alpha q
+                    A[i] = o1;
+                    C[i] = o2;
+                } else if (OP == VOP_BI_P) {
+                    // p = r + beta * (p - omega * v)     (bicgstab.hpp:49-53)
+                    o1 = first ? b[q] : fma(beta, fma(-omega, c[q], a[q]), b[q]);
+                    A[i] = o1;
+                } else if (OP == VOP_BI_S) {
+                    o1 = fma(-alpha, c[q], b[q]);                           // s = r - alpha v
+                    A[i] = o1;
+                } else if (OP == VOP_BI_XR) {
+                    // A x, B phat, C shat, E s, F t, G r
+                    if (finishing) {
+                        A[i] = fma(alpha, b[q], a[q]);                      // x += alpha phat
+                    } else {
+                        // x += omega shat + alpha phat, evaluated as the reference
+                        // build does: x + fma(alpha, phat, omega shat)
+                        o1 = a[q] + fma(alpha, b[q], omega * c[q]);
+                        o2 = fma(-omega, f[q], e[q]);                       // r = s - omega t
+                        A[i] = o1;
+                        G[i] = o2;
+                    }
+                } else if (OP == VOP_REF_CAST) {
+                    // inner right-hand side float(r64 / ||r64||); inner x = 0, r = b
+                    o2 = T(w[q] / scale);
+                    A[i] = o2;
+                    if (B) B[i] = T(0);
+                    if (C) C[i] = o2;
+                    if (E) E[i] = o2;
+                } else if (OP == VOP_REF_UPDATE) {
+                    d.x64[i] = fma(scale, double(a[q]), w[q]);              // x += ||r|| * d
+                } else if (OP == VOP_FILL) {
+                    A[i] = T(op.scalar);
+                } else if (OP == VOP_COPY) {
+                    A[i] = b[q];
+                } else if (OP == VOP_SCALE_COPY) {
+                    A[i] = T(op.scalar) * b[q];
+                }
+#pragma unroll
+                for (int j = 0; j < ND; ++j) {
+                    const T x = from[2 * j] == 1 ? o1 : from[2 * j] == 2 ? o2 : m[q][2 * j];
+                    const T y = from[2 * j + 1] == 1 ? o1 : from[2 * j + 1] == 2 ? o2 : m[q][2 * j + 1];
+                    dot[q * NV + j] += double(x * y * (by_d[j] ? dd[q] : T(1)));
+                }
             }
             if (!reduce || ng == 0) continue;
-            block_reduce<NR>(dot, s_red);
-            if (threadIdx.x == 0) {
-#pragma unroll
-                for (int q = 0; q < kVecGroup; ++q)
-                    if (q < ng)
-#pragma unroll
-                        for (int j = 0; j < kMaxDots; ++j) sv.partials[(long long)(t + q) * kMaxDots + j] = dot[q * kMaxDots + j];
+            if constexpr (ND > 0) {
+                const double sum = warp_sums<NR>(dot);
+                const int k = warp_sum_index<NR>(lane), q = k / NV;
+                if (lane % (32 / NR) == 0 && q < ng) s_part[((held + q) * (kBlock / 32) + warp) * NV + k % NV] = sum;
+                held += ng;
+                if (held > kPartTiles - kVecGroup) {
+                    flush_parts<NV>(sv, t + ng - held, held, s_part);
+                    held = 0;
+                }
             }
             tally.n += unsigned(ng);
         }
+        if (ND > 0 && held) flush_parts<NV>(sv, tb + min(te - tb, nvt) - held, held, s_part);
         t = te;
     }
     vec_publish<OP>(sv, op, tally, s_red);

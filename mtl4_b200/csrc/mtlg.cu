@@ -801,7 +801,8 @@ static int spmv_impl(mtlg_ctx* c, mtlg_csr* A, const mtlg_vec* x, mtlg_vec* y, i
     // row lengths, stream tiles otherwise
     const int kern = c->spmv_kernel != 0 ? c->spmv_kernel
                      : A->irregular ? 2
-                     : (A->n_rows > 0 && A->nnz <= int64_t(kScalarMeanRow) * A->n_rows) ? 3 : 1;
+                     : csr_short_rows(A) ? 3 : 1;
+    if (c->spmv_kernel == 1) sv.short_rows = 0;   // stream tiles asked for
     if (!pq && kern == 3) {
         const int grid = int(std::min<int64_t>((A->n_rows + kBlock - 1) / kBlock, int64_t(c->sm_count) * 16));
         if (A->n_rows == 0) return MTLG_OK;
