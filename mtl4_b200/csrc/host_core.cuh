@@ -3,6 +3,7 @@
 #include "sweep.cuh"
 #include "gridsweep.cuh"
 #include "refdot.cuh"
+#include "cgsmall.cuh"
 #include "trace.cuh"
 #include "mmio.cuh"
 
@@ -519,6 +520,28 @@ template <typename T, int XF, int ASG> int ShortShape<T, XF, ASG>::occ[3] = {0, 
     M(XF_CG_P, ASG_SET)           \
     M(XF_CG_P_JAC, ASG_SET)       \
     M(XF_JAC, ASG_SET)
+
+// k_cg_small: at most one CTA per SM, with the fewest rows per thread (1, 2 or
+// 4) that gives each its own.
+template <typename T, bool JAC>
+struct CgSmallShape {
+    static int rows(const mtlg_ctx* c, int n_tiles)   // 0: too many
+    {
+        for (int r = 1; r <= 4; r *= 2)
+            if ((n_tiles + r - 1) / r <= c->sm_count) return r;
+        return 0;
+    }
+    static int launch(mtlg_ctx* c, const SetView& sv, double* cells, int r)
+    {
+        SetView v = sv;
+        void* args[2] = {&v, &cells};
+        const void* f = r == 1 ? (const void*)k_cg_small<T, JAC, 1>
+                      : r == 2 ? (const void*)k_cg_small<T, JAC, 2> : (const void*)k_cg_small<T, JAC, 4>;
+        MTLG_CUDA(cudaLaunchCooperativeKernel(f, dim3(unsigned((sv.n_tiles + r - 1) / r)), dim3(kBlock), args, 0, c->stream));
+        c->launches++;
+        return MTLG_OK;
+    }
+};
 
 // Called once per context (kernel attributes may not change inside a stream
 // capture).

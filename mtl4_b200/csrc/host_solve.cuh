@@ -60,6 +60,7 @@ struct SolveSet {
     cudaGraphExec_t chunk_exec = nullptr;
     int chunk_kernels = 0;
     int* h_running = nullptr;       // pinned host copies of the running count
+    DBuf<double> cells;             // k_cg_small's meeting cells
     cudaEvent_t chunk_ev[2] = {nullptr, nullptr};
     ~SolveSet()
     {
@@ -605,8 +606,39 @@ inline int run_loop_chunked(SolveSet& ss, int max_iter)
     return MTLG_OK;
 }
 
-// Runs the loop until no system is running.  Default: chunked plain graphs
-// (run_loop_chunked).  loop_mode 1: one graph with a WHILE conditional node,
+// Rows per thread of the one-launch CG (k_cg_small) for this set, 0 where it
+// does not apply: one system, no or diagonal preconditioner, short regular
+// rows, whole 256-row product tiles (they are the vector passes' tiles then,
+// so the dots' partials are the same), and few enough rows that all run at
+// once.  Two kernels an iteration win again only where a pass is long against
+// its launch (beyond these sizes).  Not in the reference's summation order,
+// whose dots are whole-vector chains.
+template <typename T>
+inline int cg_small_rows(const SolveSet& ss)
+{
+    const mtlg_ctx* c = ss.ctx;
+    if (ss.solver != MTLG_CG || ss.S != 1 || ss.path == PATH_SWEEP || !ss.short_rows) return 0;
+    if (std::is_same<T, double>::value && c->red_order == 1) return 0;
+    if (c->spin_limit > 0 && c->spin_limit < kSpinLimit) return 0;   // short waits are asked for; the two-kernel loop has none
+    if (int64_t(ss.n_tiles) != (ss.in[0].A->n_rows + kTileRows - 1) / kTileRows) return 0;
+    return ss.path == PATH_JACOBI ? CgSmallShape<T, true>::rows(c, ss.n_tiles) : CgSmallShape<T, false>::rows(c, ss.n_tiles);
+}
+template <typename T>
+inline int run_cg_small(SolveSet& ss, int rows)
+{
+    mtlg_ctx* c = ss.ctx;
+    const size_t cells = size_t(cg_cells(ss.n_tiles));
+    if (!ss.cells.p) MTLG_TRY(ss.cells.alloc(c, cells));
+    MTLG_CUDA(cudaMemsetAsync(ss.cells.p, 0xFF, cells * sizeof(double), c->stream));
+    const SetView sv = ss.view(false, false);
+    if (ss.path == PATH_JACOBI) MTLG_TRY((CgSmallShape<T, true>::launch(c, sv, ss.cells.p, rows)));
+    else MTLG_TRY((CgSmallShape<T, false>::launch(c, sv, ss.cells.p, rows)));
+    MTLG_CUDA(cudaStreamSynchronize(c->stream));
+    return MTLG_OK;
+}
+
+// Runs the loop until no system is running.  Default: one launch for small CG
+// solves (run_cg_small), else chunked plain graphs (run_loop_chunked).  loop_mode 1: one graph with a WHILE conditional node,
 // one launch per solve.  If a graph cannot be built, or under loop_mode 2
 // (for profilers that do not see kernels inside graphs), the body is
 // launched directly from the host, 8 at a time.
@@ -617,7 +649,10 @@ inline int run_loop(SolveSet& ss, int max_iter)
     const int ipb = iters_per_body(ss);
     int hdr[3] = {0, 0, max_iter / ipb + 4};   // err flag, body runs, cap
     MTLG_CUDA(cudaMemcpyAsync(ss.misc.p + 1, hdr, sizeof hdr, cudaMemcpyHostToDevice, c->stream));
-    if (c->loop_mode == 0) return run_loop_chunked<T>(ss, max_iter);
+    if (c->loop_mode == 0) {
+        const int rows = cg_small_rows<T>(ss);
+        return rows > 0 ? run_cg_small<T>(ss, rows) : run_loop_chunked<T>(ss, max_iter);
+    }
     if (c->loop_mode == 1) MTLG_TRY(build_graph<T>(ss));   // loop_mode 2: direct launches (profilers)
     if (c->loop_mode == 1 && ss.exec) {
         MTLG_CUDA(cudaGraphLaunch(ss.exec, c->stream));
