@@ -49,7 +49,7 @@ PEAKS = ROOT / "MEASURED_PEAKS.json"
 # DRAM bytes (read + write) of one FP32 ILU(0) apply (the L and U sweep
 # launches) from one ncu capture of this workload, per sweep kernel
 TRAFFIC_PER_APPLY = {"chunked": 210_680_000,   # k_sweep_chunk: 105.1 MB (L) + 105.5 MB (U)
-                     "grid": 104_306_000}      # k_sweep_grid: 52.28 MB (L) + 52.03 MB (U)
+                     "grid": 95_106_000}       # k_sweep_grid: 47.58 MB (L) + 47.53 MB (U)
 FALLBACK_HBM = 6650.0
 
 
@@ -525,8 +525,8 @@ def main():
     nnz_off = len(Lv) + (len(Uv) - n)
     if plan["kernel"] == "grid":
         # grid layout (no indices): entry values and one multiplier per row,
-        # right-hand side read, result written, the other vector reset, per sweep
-        bytes_apply = 4 * nnz_off + 2 * 4 * n + 2 * 3 * 4 * n
+        # right-hand side read, result written, per sweep
+        bytes_apply = 4 * nnz_off + 2 * 4 * n + 2 * 2 * 4 * n
         sweep_kernel = "k_sweep_grid<float,float> (ILU(0) L and U sweeps, one apply)"
     else:
         bytes_apply = 8 * nnz_off + 2 * 12 * n + 4 * n * 4

@@ -531,13 +531,21 @@ struct CgSmallShape {
             if ((n_tiles + r - 1) / r <= c->sm_count) return r;
         return 0;
     }
-    static int launch(mtlg_ctx* c, const SetView& sv, double* cells, int r)
+    // `ran` false: this device or context cannot run that many CTAs at once.
+    static int launch(mtlg_ctx* c, const SetView& sv, double* cells, int r, bool& ran)
     {
         SetView v = sv;
         void* args[2] = {&v, &cells};
         const void* f = r == 1 ? (const void*)k_cg_small<T, JAC, 1>
                       : r == 2 ? (const void*)k_cg_small<T, JAC, 2> : (const void*)k_cg_small<T, JAC, 4>;
-        MTLG_CUDA(cudaLaunchCooperativeKernel(f, dim3(unsigned((sv.n_tiles + r - 1) / r)), dim3(kBlock), args, 0, c->stream));
+        const cudaError_t e =
+            cudaLaunchCooperativeKernel(f, dim3(unsigned((sv.n_tiles + r - 1) / r)), dim3(kBlock), args, 0, c->stream);
+        ran = e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported;
+        if (!ran) {
+            cudaGetLastError();
+            return MTLG_OK;
+        }
+        MTLG_CUDA(e);
         c->launches++;
         return MTLG_OK;
     }
@@ -661,11 +669,14 @@ inline int launch_vec(mtlg_ctx* c, cudaStream_t st, const SetView& sv, const Vec
     // one CTA per run of tiles, vec_ctas_per_sm per SM at most (each CTA
     // publishes its dot tally with one atomic on the system's counter)
     dim3 g(std::min(sv.n_tiles, c->vec_ctas_per_sm * c->sm_count)), b(kBlock);
-    if (op.ndot > 2) {
-        set_error("a vector pass reduces at most two dots");
+    const bool dots = op.op == VOP_DOT || op.op == VOP_CG_UPDATE || op.op == VOP_BI_S || op.op == VOP_BI_XR || op.op == VOP_REF_CAST;
+    if (op.ndot > (dots ? 2 : 0)) {
+        set_error("vector pass %d with %d dots", op.op, op.ndot);
         return MTLG_ERR_NOT_SUPPORTED;
     }
     switch (op.op) {
+#define MTLG_VEC_PLAIN(OP) \
+    case OP: k_vec<T, OP, 0><<<g, b, 0, st>>>(sv, op); break;
 #define MTLG_VEC_CASE(OP)                                          \
     case OP:                                                       \
         if (op.ndot == 0) k_vec<T, OP, 0><<<g, b, 0, st>>>(sv, op);      \
@@ -673,17 +684,18 @@ inline int launch_vec(mtlg_ctx* c, cudaStream_t st, const SetView& sv, const Vec
         else k_vec<T, OP, 2><<<g, b, 0, st>>>(sv, op);                   \
         break;
         MTLG_VEC_CASE(VOP_DOT)
-        MTLG_VEC_CASE(VOP_AXPY)
+        MTLG_VEC_PLAIN(VOP_AXPY)
         MTLG_VEC_CASE(VOP_CG_UPDATE)
-        MTLG_VEC_CASE(VOP_BI_P)
+        MTLG_VEC_PLAIN(VOP_BI_P)
         MTLG_VEC_CASE(VOP_BI_S)
         MTLG_VEC_CASE(VOP_BI_XR)
         MTLG_VEC_CASE(VOP_REF_CAST)
-        MTLG_VEC_CASE(VOP_REF_UPDATE)
-        MTLG_VEC_CASE(VOP_FILL)
-        MTLG_VEC_CASE(VOP_COPY)
-        MTLG_VEC_CASE(VOP_SCALE_COPY)
+        MTLG_VEC_PLAIN(VOP_REF_UPDATE)
+        MTLG_VEC_PLAIN(VOP_FILL)
+        MTLG_VEC_PLAIN(VOP_COPY)
+        MTLG_VEC_PLAIN(VOP_SCALE_COPY)
 #undef MTLG_VEC_CASE
+#undef MTLG_VEC_PLAIN
     default:
         set_error("unsupported vector op %d", op.op);
         return MTLG_ERR_NOT_SUPPORTED;

@@ -624,15 +624,15 @@ inline int cg_small_rows(const SolveSet& ss)
     return ss.path == PATH_JACOBI ? CgSmallShape<T, true>::rows(c, ss.n_tiles) : CgSmallShape<T, false>::rows(c, ss.n_tiles);
 }
 template <typename T>
-inline int run_cg_small(SolveSet& ss, int rows)
+inline int run_cg_small(SolveSet& ss, int rows, bool& ran)
 {
     mtlg_ctx* c = ss.ctx;
     const size_t cells = size_t(cg_cells(ss.n_tiles));
     if (!ss.cells.p) MTLG_TRY(ss.cells.alloc(c, cells));
     MTLG_CUDA(cudaMemsetAsync(ss.cells.p, 0xFF, cells * sizeof(double), c->stream));
     const SetView sv = ss.view(false, false);
-    if (ss.path == PATH_JACOBI) MTLG_TRY((CgSmallShape<T, true>::launch(c, sv, ss.cells.p, rows)));
-    else MTLG_TRY((CgSmallShape<T, false>::launch(c, sv, ss.cells.p, rows)));
+    if (ss.path == PATH_JACOBI) MTLG_TRY((CgSmallShape<T, true>::launch(c, sv, ss.cells.p, rows, ran)));
+    else MTLG_TRY((CgSmallShape<T, false>::launch(c, sv, ss.cells.p, rows, ran)));
     MTLG_CUDA(cudaStreamSynchronize(c->stream));
     return MTLG_OK;
 }
@@ -651,7 +651,9 @@ inline int run_loop(SolveSet& ss, int max_iter)
     MTLG_CUDA(cudaMemcpyAsync(ss.misc.p + 1, hdr, sizeof hdr, cudaMemcpyHostToDevice, c->stream));
     if (c->loop_mode == 0) {
         const int rows = cg_small_rows<T>(ss);
-        return rows > 0 ? run_cg_small<T>(ss, rows) : run_loop_chunked<T>(ss, max_iter);
+        bool ran = false;
+        if (rows > 0) MTLG_TRY(run_cg_small<T>(ss, rows, ran));
+        return ran ? MTLG_OK : run_loop_chunked<T>(ss, max_iter);
     }
     if (c->loop_mode == 1) MTLG_TRY(build_graph<T>(ss));   // loop_mode 2: direct launches (profilers)
     if (c->loop_mode == 1 && ss.exec) {
