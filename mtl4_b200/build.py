@@ -10,7 +10,7 @@ SRC = PKG / "csrc"
 OUT = PKG / "libmtl4_b200.so"
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
-         "-Xcompiler", "-fPIC", "-shared", "-split-compile=0"]
+         "-Xcompiler", "-fPIC", "-shared"]
 
 
 def sources():
