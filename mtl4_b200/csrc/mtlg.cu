@@ -775,6 +775,30 @@ static int spmv_impl(mtlg_ctx* c, mtlg_csr* A, const mtlg_vec* x, mtlg_vec* y, i
     }
     const bool f32 = x->dtype == MTLG_F32;
     if (f32) MTLG_TRY(ensure_f32_values(A));
+    const int asg = assign == MTLG_ASSIGN ? ASG_SET : (assign == MTLG_PLUS ? ASG_ADD : ASG_SUB);
+    // auto: thread per row for short regular rows, warp tasks for irregular
+    // row lengths, stream tiles otherwise
+    const int kern = c->spmv_kernel != 0 ? c->spmv_kernel
+                     : A->irregular ? 2
+                     : csr_short_rows(A) ? 3 : 1;
+    // (these two take their operands as arguments: no descriptor to copy first)
+    if (!pq && kern == 3) {
+        const int grid = int(std::min<int64_t>((A->n_rows + kBlock - 1) / kBlock, int64_t(c->sm_count) * 16));
+        if (A->n_rows == 0) return MTLG_OK;
+        const void* va = f32 ? (const void*)A->v32.p : (const void*)A->v64.p;
+#define MTLG_SCALAR(T, ASG) k_spmv_scalar<T, ASG><<<grid, kBlock, 0, c->stream>>>(int(A->n_rows), A->rp.p, A->ci.p, (const T*)va, (const T*)x->p, (T*)y->p)
+        if (f32) { if (asg == ASG_SET) MTLG_SCALAR(float, ASG_SET); else if (asg == ASG_ADD) MTLG_SCALAR(float, ASG_ADD); else MTLG_SCALAR(float, ASG_SUB); }
+        else { if (asg == ASG_SET) MTLG_SCALAR(double, ASG_SET); else if (asg == ASG_ADD) MTLG_SCALAR(double, ASG_ADD); else MTLG_SCALAR(double, ASG_SUB); }
+#undef MTLG_SCALAR
+        c->launches++;
+        MTLG_CUDA(cudaGetLastError());
+        return MTLG_OK;
+    }
+    const bool warp = !pq && kern == 2;
+    if (warp) {
+        if (f32) return launch_spmv_rows<float>(c, A, x->p, y->p, asg);
+        return launch_spmv_rows<double>(c, A, x->p, y->p, asg);
+    }
     SetView sv;
     MTLG_TRY(csr_op_set(A, sv));
     SysDesc d;
@@ -796,30 +820,7 @@ static int spmv_impl(mtlg_ctx* c, mtlg_csr* A, const mtlg_vec* x, mtlg_vec* y, i
         set_kinds(op, RK_LDOT4);
         op.fin = FIN_STORE;
     }
-    const int asg = assign == MTLG_ASSIGN ? ASG_SET : (assign == MTLG_PLUS ? ASG_ADD : ASG_SUB);
-    // auto: thread per row for short regular rows, warp tasks for irregular
-    // row lengths, stream tiles otherwise
-    const int kern = c->spmv_kernel != 0 ? c->spmv_kernel
-                     : A->irregular ? 2
-                     : csr_short_rows(A) ? 3 : 1;
     if (c->spmv_kernel == 1) sv.short_rows = 0;   // stream tiles asked for
-    if (!pq && kern == 3) {
-        const int grid = int(std::min<int64_t>((A->n_rows + kBlock - 1) / kBlock, int64_t(c->sm_count) * 16));
-        if (A->n_rows == 0) return MTLG_OK;
-        const void* va = f32 ? (const void*)A->v32.p : (const void*)A->v64.p;
-#define MTLG_SCALAR(T, ASG) k_spmv_scalar<T, ASG><<<grid, kBlock, 0, c->stream>>>(int(A->n_rows), A->rp.p, A->ci.p, (const T*)va, (const T*)x->p, (T*)y->p)
-        if (f32) { if (asg == ASG_SET) MTLG_SCALAR(float, ASG_SET); else if (asg == ASG_ADD) MTLG_SCALAR(float, ASG_ADD); else MTLG_SCALAR(float, ASG_SUB); }
-        else { if (asg == ASG_SET) MTLG_SCALAR(double, ASG_SET); else if (asg == ASG_ADD) MTLG_SCALAR(double, ASG_ADD); else MTLG_SCALAR(double, ASG_SUB); }
-#undef MTLG_SCALAR
-        c->launches++;
-        MTLG_CUDA(cudaGetLastError());
-        return MTLG_OK;
-    }
-    const bool warp = !pq && kern == 2;
-    if (warp) {
-        if (f32) return launch_spmv_rows<float>(c, A, x->p, y->p, asg);
-        return launch_spmv_rows<double>(c, A, x->p, y->p, asg);
-    }
     if (f32) MTLG_TRY(launch_spmv<float>(c, c->stream, sv, op, XF_PLAIN, asg));
     else MTLG_TRY(launch_spmv<double>(c, c->stream, sv, op, XF_PLAIN, asg));
     MTLG_CUDA(cudaGetLastError());
