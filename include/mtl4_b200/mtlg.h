@@ -157,8 +157,8 @@ int64_t mtlg_ctx_kernel_launches(mtlg_ctx* ctx);
  * "grid_sweep" (1, default: factors whose pattern is a 5- or 7-point grid
  * stencil in natural order get, at set-up, a layout of x-lines per lane and
  * are swept by the grid kernel when sweep_kernel is 0; 0: chunked or flat
- * only), "grid_warps" (compute warps per grid-sweep CTA: 4 or 8; 0,
- * default: 8 where the shared memory fits, else 4),
+ * only), "grid_warps" (compute warps per grid-sweep CTA: 4 or 8, where the
+ * shared memory fits; 0, default: 4),
  * "chunk_rows" (rows per chunk of preconditioners created afterwards; 0:
  * 16384 for FP32 factors, 8192 for FP64), "sweep_cluster" (CTAs per
  * thread-block cluster of the chunked sweeps, whose neighbouring chunks
@@ -326,8 +326,8 @@ int mtlg_pc_levels(const mtlg_pc* P, int* levels_L, int* levels_U);
  * L, CTAs resident at once, shared memory per CTA (bytes), compute threads
  * per CTA, entries per row (register bucket), rows and entries per staged
  * segment.  Grid sweeps (grid-stencil factors): 0, 0, CTAs resident at
- * once, shared memory per CTA, compute threads per CTA (two receiver warps
- * more), entries per row, tiles of L, steps per warp unit.  All zero when
+ * once, shared memory per CTA, compute threads per CTA (as many helper threads
+ * and two receiver warps more), entries per row, tiles of L, steps per warp unit.  All zero when
  * the flat level-order sweeps run instead.  Not part of the reference's
  * interface (introspection for tuning). */
 int mtlg_pc_sweep_plan(mtlg_ctx* ctx, mtlg_pc* P, int dtype, int32_t* out8);
