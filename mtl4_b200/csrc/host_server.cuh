@@ -478,6 +478,9 @@ int mtlg_server_step(mtlg_server* S)
             MTLG_CUDA(cudaMemcpy(ss.misc.p + 1, &z, sizeof z, cudaMemcpyHostToDevice));
             MTLG_CUDA(cudaMemset(ss.tickets.p, 0, 8 * sizeof(int)));
             MTLG_TRY(reset_set_sweep_buffers(ss));
+            // rows half handed over between tiles or chunks belong to the sweep that expired
+            for (int s = 0; s < ss.S; ++s)
+                if (E.slot_req[s] >= 0) MTLG_TRY(pc_reset_sweep_state(S->reqs[E.slot_req[s]]->P));
         }
     }
     // 2. admit queued requests while slots and memory allow
