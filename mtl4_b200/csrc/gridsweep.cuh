@@ -28,8 +28,8 @@
 // What bounds it: the dependency chain (nx + ny + nz steps and the hand-offs
 // between warps and tiles), not bytes; a step costs one shuffle, a row's
 // arithmetic and the shared-memory accesses that feed it.  Measured (one
-// B200, apply = L + U sweep, queued): FP32 ILU(0) 128^3 439 -> 230 us, 2048^2
-// 1,990 -> 773 us, FP64 128^3 773 -> 366 us against the previous kernel (one
+// B200, apply = L + U sweep, queued): FP32 ILU(0) 128^3 439 -> 225 us, 2048^2
+// 1,990 -> 692 us, FP64 128^3 773 -> 304 us against the previous kernel (one
 // warp per 32 lines and plane, every lane moving its own line's right-hand
 // sides, results and resets: 32 sectors per instruction, ~300 ns a step).
 // Tiles are taken through one ticket in an order in which every tile a tile
