@@ -35,6 +35,7 @@ struct SolveSet {
     DBuf<SysState> st;
     int n_tiles = 0;
     int short_rows = 0;   // every system's rows are short and regular
+    bool whole_tiles = false;   // the product's tiles are the vector passes': kTileRows rows each but a system's last
     DBuf<Tile> tiles;
     DBuf<int> stb;
     DBuf<double> partials;
@@ -156,6 +157,11 @@ inline int build_set(mtlg_ctx* c, SolveSet& ss)
             for (int s = 0; s < ss.S; ++s) MTLG_TRY(ensure_flat(const_cast<mtlg_pc*>(ss.in[s].P)));
     }
     ss.n_tiles = int(tiles.size());
+    ss.whole_tiles = !tiles.empty();
+    for (const Tile& t : tiles)
+        if (t.kind != TILE_STREAM || t.row_begin % kTileRows != 0 ||
+            t.row_end != std::min<int64_t>(t.row_begin + kTileRows, ss.in[t.sys].A->n_rows))
+            ss.whole_tiles = false;
     MTLG_TRY(ss.tiles.upload(c, tiles.data(), std::max<size_t>(1, tiles.size())));
     MTLG_TRY(ss.stb.upload(c, stb.data(), stb.size()));
     MTLG_TRY(ss.partials.alloc(c, size_t(std::max(1, ss.n_tiles)) * kMaxDots));
@@ -609,8 +615,9 @@ inline int run_loop_chunked(SolveSet& ss, int max_iter)
 // Rows per thread of the one-launch CG (k_cg_small) for this set, 0 where it
 // does not apply: one system, no or diagonal preconditioner, short regular
 // rows, whole 256-row product tiles (they are the vector passes' tiles then,
-// so the dots' partials are the same), and few enough rows that all run at
-// once.  Two kernels an iteration win again only where a pass is long against
+// so the dots' partials are the same; tiles that kTileNnz entries cut short
+// add the same products up in another grouping), and few enough rows that all
+// run at once.  Two kernels an iteration win again only where a pass is long against
 // its launch (beyond these sizes).  Not in the reference's summation order,
 // whose dots are whole-vector chains.
 template <typename T>
@@ -620,7 +627,7 @@ inline int cg_small_rows(const SolveSet& ss)
     if (ss.solver != MTLG_CG || ss.S != 1 || ss.path == PATH_SWEEP || !ss.short_rows) return 0;
     if (std::is_same<T, double>::value && c->red_order == 1) return 0;
     if (c->spin_limit > 0 && c->spin_limit < kSpinLimit) return 0;   // short waits are asked for; the two-kernel loop has none
-    if (int64_t(ss.n_tiles) != (ss.in[0].A->n_rows + kTileRows - 1) / kTileRows) return 0;
+    if (!ss.whole_tiles) return 0;
     return ss.path == PATH_JACOBI ? CgSmallShape<T, true>::rows(c, ss.n_tiles) : CgSmallShape<T, false>::rows(c, ss.n_tiles);
 }
 template <typename T>
