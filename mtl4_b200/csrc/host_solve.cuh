@@ -750,17 +750,19 @@ inline int run_refine(SolveSet& ss, const mtlg_refine_params& rp)
     nb.fin = FIN_REF_NB;
     MTLG_TRY(launch_vec<double>(c, c->stream, v64, nb));
     for (int outer = 0; outer <= rp.max_outer; ++outer) {
-        MTLG_CUDA(cudaMemsetAsync(ss.misc.p, 0, sizeof(int), c->stream));
+        MTLG_CUDA(cudaMemsetAsync(ss.misc.p, 0, (outer == 0 ? 2 : 1) * sizeof(int), c->stream));
         SpmvOp r = spmv_op_default();
         r.x = SLOT_X; r.w = SLOT_B; r.y = 0;
         set_dot(r, 0, OPND_Y, OPND_Y);
         r.fin = FIN_REF_OUTER;
         r.skip = SKIP_OUTER;
         MTLG_TRY(launch_spmv<double>(c, c->stream, v64, r, XF_PLAIN, ASG_WMINUS));
-        int running = 0;
-        MTLG_CUDA(cudaMemcpyAsync(&running, ss.misc.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        // systems running; whether a wait of the last inner loop expired (the
+        // next loop would clear the flag, and sweep on rows half handed over)
+        int head[2] = {0, 0};
+        MTLG_CUDA(cudaMemcpyAsync(head, ss.misc.p, sizeof head, cudaMemcpyDeviceToHost, c->stream));
         MTLG_CUDA(cudaStreamSynchronize(c->stream));
-        if (running == 0) break;
+        if (head[0] == 0 || head[1] != 0) break;
         if (ss.solver == MTLG_CG) MTLG_TRY(cg_init<float>(ss, c->stream, v32, true));
         else MTLG_TRY(bicg_init<float>(ss, c->stream, v32, true));
         MTLG_TRY(run_loop<float>(ss, rp.max_inner));
