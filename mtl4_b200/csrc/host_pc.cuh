@@ -1228,6 +1228,7 @@ struct mtlg_pc {
     DBuf<double> inv_dia;           // FP64 pivots (ILU: 1/u_ii, IC: 1/sqrt(u_ii))
     DBuf<unsigned char> tmp;        // sentinel-filled temporary (n x 8 bytes)
     bool tmp_used = false;          // a grid sweep left values in tmp: flat sweeps need the sentinel back first
+    bool queued = false;            // queued applies since the expired-wait flag was last read
     DBuf<int> tickets;              // self-resetting work tickets
     DBuf<SysDesc> desc;
     DBuf<SysState> st;
@@ -1318,6 +1319,27 @@ inline int pc_reset_sweep_state(mtlg_pc* P)
     P->tmp_used = false;
     return MTLG_OK;
 }
+
+// Reads the flag of this preconditioner's applies (waits for the stream);
+// after an expired wait everything is reset and the timeout reported.
+inline int pc_check_expired(mtlg_pc* P)
+{
+    mtlg_ctx* c = P->ctx;
+    int err = 0;
+    MTLG_CUDA(cudaMemcpyAsync(&err, P->misc.p + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    MTLG_CUDA(cudaStreamSynchronize(c->stream));
+    P->queued = false;
+    if (!err) return MTLG_OK;
+    int z = 0;
+    MTLG_CUDA(cudaMemcpy(P->misc.p + 1, &z, sizeof z, cudaMemcpyHostToDevice));
+    MTLG_CUDA(cudaMemset(P->tickets.p, 0, 8 * sizeof(int)));
+    MTLG_TRY(pc_reset_sweep_state(P));
+    set_error("triangular sweep dependency wait expired");
+    return MTLG_ERR_TIMEOUT;
+}
+// Before a solve uses P's factors: a queued apply that expired has left rows
+// half handed over in them, which the solve's sweeps would take for theirs.
+inline int pc_settle_queued(mtlg_pc* P) { return P && P->queued ? pc_check_expired(P) : MTLG_OK; }
 
 inline int pc_setup_single_set(mtlg_pc* P)
 {

@@ -173,20 +173,10 @@ int pc_sweeps(mtlg_pc* P, const mtlg_vec* x, mtlg_vec* y)
     }
     MTLG_CUDA(cudaGetLastError());
     // queued applies (pc_apply_sync = 0): an expired wait stays flagged on the
-    // device and is reported by the next synchronous apply of this preconditioner
-    if (!c->pc_apply_sync) return MTLG_OK;
-    int err = 0;
-    MTLG_CUDA(cudaMemcpyAsync(&err, P->misc.p + 1, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    MTLG_CUDA(cudaStreamSynchronize(c->stream));
-    if (err) {
-        int z = 0;
-        MTLG_CUDA(cudaMemcpy(P->misc.p + 1, &z, sizeof z, cudaMemcpyHostToDevice));
-        MTLG_CUDA(cudaMemset(P->tickets.p, 0, 8 * sizeof(int)));
-        MTLG_TRY(pc_reset_sweep_state(P));
-        set_error("triangular sweep dependency wait expired");
-        return MTLG_ERR_TIMEOUT;
-    }
-    return MTLG_OK;
+    // device and is reported by the next synchronous apply or solve with this
+    // preconditioner
+    P->queued = true;
+    return c->pc_apply_sync ? pc_check_expired(P) : MTLG_OK;
 }
 
 // SpMV on raw device pointers of the CSR's size (GMRES workspace vectors);
@@ -1213,6 +1203,7 @@ int mtlg_solve(mtlg_ctx* c, int solver, mtlg_csr* A, mtlg_pc* L, mtlg_pc* R, mtl
         MTLG_TRY(build_set(c, *ss));
         slot = std::move(ss);
     }
+    MTLG_TRY(pc_settle_queued(L));
     SolveSet& ss = *slot;
     SysInput& si = ss.in[0];
     si.x = x->p;
@@ -1326,6 +1317,7 @@ int mtlg_refine_solve(mtlg_ctx* c, int solver, mtlg_csr* A, mtlg_pc* P, mtlg_vec
         MTLG_TRY(build_set(c, *ss));
         slot = std::move(ss);
     }
+    MTLG_TRY(pc_settle_queued(P));
     SolveSet& ss = *slot;
     ss.in[0].x = x->p;
     ss.in[0].b = b->p;

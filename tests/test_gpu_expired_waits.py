@@ -1,5 +1,7 @@
-"""Waits of the grid sweeps that run out inside a refinement: it stops there,
-reports the timeout and leaves the preconditioner usable."""
+"""Waits of the grid sweeps that run out where nobody looks at once: inside a
+refinement that goes on, and in queued applies.  The rows half handed over
+between tiles belong to the preconditioner, so the next user of it has to
+learn of the expiry; afterwards everything is the bits of before."""
 import contextlib
 
 import numpy as np
@@ -58,3 +60,35 @@ def test_refinement_stops_at_the_inner_loop_whose_wait_ran_out(ctx):
         expired, launches, _ = refine(Pw, 8)
     assert expired and launches <= one_outer
     assert np.array_equal(itl.solve(Pw, v).numpy(), want)
+
+
+@pytest.mark.parametrize("solver", ["bicgstab", "refine"])
+def test_queued_apply_that_ran_out_is_reported_by_a_solve(ctx, solver):
+    from mtl4_b200 import _lib, itl, mtl
+    A = P.convdiff_3d(32)
+    st = np.float32 if solver == "refine" else np.float64
+    Ad = mtl.compressed2D.from_problem(A, ctx)
+    Pc = itl.pc.ilu_0(Ad, st)
+    b = mtl.dense_vector(P.random_rhs(A.n_rows, 1), np.float64, ctx)
+    v, y = mtl.dense_vector(P.random_rhs(A.n_rows, 2).astype(st), st, ctx), mtl.dense_vector(A.n_rows, st, ctx)
+
+    def solve():
+        x = mtl.dense_vector(A.n_rows, np.float64, ctx)
+        if solver == "refine":
+            it = itl.refine("bicgstab", Ad, x, b, Pc)
+        else:
+            it = itl.basic_iteration(b, 500, 1e-8)
+            itl.bicgstab(Ad, x, b, Pc, it)
+        return it.iterations(), x.numpy()
+
+    n0, x0 = solve()
+    with tuning(ctx, pc_apply_sync=0):
+        itl.solve(Pc, v, y)
+        assert solve()[0] == n0   # queued applies that ran through
+        with tuning(ctx, spin_limit=1):
+            itl.solve(Pc, v, y)
+    with pytest.raises(_lib.device_timeout):
+        solve()
+    for _ in range(2):
+        n1, x1 = solve()
+        assert n1 == n0 and np.array_equal(x1, x0)
