@@ -194,11 +194,18 @@ __device__ __forceinline__ void grid_acquire() { asm volatile("fence.acq_rel.cta
 // Whether a warp's bounded wait ends without its value: after lim polls
 // (recorded as a timeout), or when another wait has expired.  Decided by all
 // lanes together, every lane having counted the same polls: the waits below
-// and what follows them use warp-wide votes.
+// and what follows them use warp-wide votes.  A wait of more than kGridQuick
+// polls (0.1 ms in shared memory) naps between them: it leaves the issue slots
+// to the others, and the default limit stays about half a second whatever a
+// poll costs (2^20 polls of shared memory alone: some 40 ms).
+constexpr long long kGridQuick = 4096;
 __device__ __forceinline__ bool grid_give_up(long long& spins, int* err, long long lim)
 {
     const bool over = ++spins > (lim > 0 ? lim : kSpinLimit);
-    if (!over && (spins & 255) != 0) return false;
+    if (!over && (spins & 255) != 0) {
+        if (spins > kGridQuick) __nanosleep(500);
+        return false;
+    }
     if (over) atomicExch(err, 1);
     return __any_sync(0xffffffffu, over || *(volatile int*)err);
 }
@@ -533,10 +540,12 @@ __device__ __forceinline__ void grid_help(const S* src, unsigned stage, const T*
 // of rows into its ring (columns col + WD g) with the sentinel back in its
 // place, and publishes the count of rows there (group g is read by compute
 // warp g * step: its count at `reader`, its slot's at `count`).  A thread holds VN elements
-// (16 bytes) of a row, so a group's poll is one coalesced load or a few.
+// (16 bytes) of a row, so a group's poll is one coalesced load or a few; sleep_ns
+// (the context's "sweep_sleep_ns") passes between polls that brought nothing.
 template <typename T, int WD, int NG>
 __device__ __forceinline__ void grid_receive(T* const (&src)[NG], int total, unsigned ring, int col, unsigned count,
-                                             unsigned reader, int step, int slack, int lane, int* err, long long spin)
+                                             unsigned reader, int step, int slack, int lane, int* err, long long spin,
+                                             int sleep_ns)
 {
     constexpr int VN = WD * int(sizeof(T)) >= 16 ? 16 / int(sizeof(T)) : 1;   // elements per thread
     constexpr int TR = WD / VN;                                              // threads per row
@@ -597,7 +606,12 @@ __device__ __forceinline__ void grid_receive(T* const (&src)[NG], int total, uns
                 if (c[g] >= total) left &= ~(1u << g);
             }
         }
-        if (!moved && grid_give_up(spins, err, spin)) break;
+        if (moved) {
+            spins = 0;   // the limit is one wait's, not the tile's
+            continue;
+        }
+        if (grid_give_up(spins, err, spin)) break;
+        if (sleep_ns > 0) __nanosleep(sleep_ns);
     }
     __syncwarp();
     // after an expired wait nobody waits on these rows any more
@@ -610,7 +624,7 @@ __device__ __forceinline__ void grid_receive(T* const (&src)[NG], int total, uns
 // them alive (96 registers and 370 bytes of spills instead of 80 and none).
 template <typename T, typename S, int NW, int NS, bool FAR, bool REV, int OPK>
 __device__ __noinline__ void grid_tile(const TriFactor& F, int n, const T* vin, T* vout, int ty, int tz,
-                                          const GridSmem& sm, int warp, int lane, int* err, long long spin)
+                                          const GridSmem& sm, int warp, int lane, int* err, long long spin, int sleep_ns)
 {
     typedef GridShapeOf<NW, NS> Sh;
     constexpr unsigned P = grid_pitch<T>() * sizeof(T), TS = sizeof(T);
@@ -632,7 +646,8 @@ __device__ __noinline__ void grid_tile(const TriFactor& F, int n, const T* vin, 
                 const int ju = ty * Sh::WY + a;
                 src[a] = tz > 0 && ju < njb ? zh + (size_t(tz - 1) * njb + ju) * total * Sh::LY : nullptr;
             }
-            grid_receive<T, Sh::LY, Sh::WY>(src, total, rring, 0, sm.slots + 4, sm.prog, 1, Sh::LZ - 1, lane, err, spin);
+            grid_receive<T, Sh::LY, Sh::WY>(src, total, rring, 0, sm.slots + 4, sm.prog, 1, Sh::LZ - 1, lane, err, spin,
+                                               sleep_ns);
         }
         return;
     }
@@ -643,7 +658,8 @@ __device__ __noinline__ void grid_tile(const TriFactor& F, int n, const T* vin, 
             const int ku = tz * Sh::WZ + a;
             src[a] = ty > 0 && ku < nkb ? yh + (size_t(ty - 1) * nkb + ku) * total * Sh::LZ : nullptr;
         }
-        grid_receive<T, Sh::LZ, Sh::WZ>(src, total, rring, Sh::ZCOLS, sm.slots, sm.prog, Sh::WY, Sh::LY - 1, lane, err, spin);
+        grid_receive<T, Sh::LZ, Sh::WZ>(src, total, rring, Sh::ZCOLS, sm.slots, sm.prog, Sh::WY, Sh::LY - 1, lane, err, spin,
+                                           sleep_ns);
         return;
     }
     const int w = warp % NW, wy = w % Sh::WY, wz = w / Sh::WY;
@@ -761,14 +777,14 @@ __global__ void __launch_bounds__(32 * (2 * NW + kGridRecvWarps), 1) k_sweep_gri
                 for (int r = ty * kGridDiagRows + tid; r < e; r += NTH) vout[r] = unsentinel(T(W(vin[r]) * W(dia[r])));
             } else if (ns == 3) {
                 if (OPK != kGridSweep || F.gperm == kGridFar3)
-                    grid_tile<T, S, NW, 3, true, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin);
+                    grid_tile<T, S, NW, 3, true, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin, op.sleep_ns);
                 else
-                    grid_tile<T, S, NW, 3, false, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin);
+                    grid_tile<T, S, NW, 3, false, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin, op.sleep_ns);
             } else {
                 if (OPK != kGridSweep || F.gperm == kGridFar2)
-                    grid_tile<T, S, NW, 2, true, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin);
+                    grid_tile<T, S, NW, 2, true, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin, op.sleep_ns);
                 else
-                    grid_tile<T, S, NW, 2, false, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin);
+                    grid_tile<T, S, NW, 2, false, REV, OPK>(F, n, vin, vout, ty, tz, sm, warp, lane, sv.err, sv.spin, op.sleep_ns);
             }
             __syncthreads();   // every warp has read its block count
             if (tid < NW && ns > 0) {
