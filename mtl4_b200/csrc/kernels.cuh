@@ -402,12 +402,17 @@ __device__ __forceinline__ void stage_tile(const Tile& t, const int* rp, const i
 // entries) is summed by the whole CTA straight from global memory.
 // Publishes a CTA's tally of a system's finished SpMV tiles; the CTA that
 // completes the system gathers its partials and finalizes.
-template <typename OpT>
+// ALL: all kMaxDots partials are there and are gathered, whatever op.ndot is.
+// (k_spmv: choosing among the three gathers costs its 80 registers 110 bytes
+// of spills in FP32 and 100 more in FP64, on 14 random entries a row 114 us
+// instead of 85 and 140 instead of 115.)
+template <bool ALL, typename OpT>
 __device__ __forceinline__ void spmv_publish(const SetView& sv, const OpT& op, TileTally& tally, double* s_red)
 {
     if (publish_tally(sv, tally)) {
         double tot[kMaxDots];
-        gather_partials(sv, tally.sys, op.ndot, tot, s_red);
+        if (ALL) gather_dots<kMaxDots>(sv, sv.sys_tile_begin[tally.sys], sv.sys_tile_begin[tally.sys + 1], tot, s_red);
+        else gather_partials(sv, tally.sys, op.ndot, tot, s_red);
         if (threadIdx.x == 0) finalize(sv, op.fin, tally.sys, tot);
     }
 }
@@ -458,7 +463,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_spmv(SetView sv, SpmvOp op)
         const Tile tile = cur;
         const int sys = tile.sys;
         if (op.fin != FIN_NONE && sys != tally.sys) {
-            spmv_publish(sv, op, tally, s_red);
+            spmv_publish<true>(sv, op, tally, s_red);
             tally.sys = sys;
         }
         const SysDesc& d = sv.desc[sys];
@@ -565,7 +570,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_spmv(SetView sv, SpmvOp op)
         nxt = nn;
     }
     cp_async_wait_0();
-    if (op.fin != FIN_NONE) spmv_publish(sv, op, tally, s_red);
+    if (op.fin != FIN_NONE) spmv_publish<true>(sv, op, tally, s_red);
 }
 
 // ---------------------------------------------------------------- SpMV, thread per row
@@ -595,7 +600,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_spmv_short(SetView sv, SpmvOp op)
         const int sys = sv.n_sys == 1 ? 0 : sv.tiles[t].sys;
         const int te = sv.n_sys == 1 ? t_end : min(t_end, sv.sys_tile_begin[sys + 1]);   // this system's tiles in the CTA's run
         if (op.fin != FIN_NONE && sys != tally.sys) {
-            spmv_publish(sv, op, tally, s_red);
+            spmv_publish<false>(sv, op, tally, s_red);
             tally.sys = sys;
         }
         const SysState& s = sv.st[sys];
@@ -667,7 +672,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_spmv_short(SetView sv, SpmvOp op)
             tally.n += unsigned(held);
         }
     }
-    if (op.fin != FIN_NONE) spmv_publish(sv, op, tally, s_red);
+    if (op.fin != FIN_NONE) spmv_publish<false>(sv, op, tally, s_red);
 }
 
 // ---------------------------------------------------------------- SpMV, warp tasks
