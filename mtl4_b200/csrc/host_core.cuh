@@ -675,6 +675,12 @@ inline int launch_vec(mtlg_ctx* c, cudaStream_t st, const SetView& sv, const Vec
         set_error("vector pass %d with %d dots", op.op, op.ndot);
         return MTLG_ERR_NOT_SUPPORTED;
     }
+    // k_vec's dots are x y or x D y of two vectors (or ones)
+    for (int j = 0; j < op.ndot; ++j)
+        if (op.da[j] == OPND_D || op.db[j] == OPND_D || (op.dc[j] != OPND_ONE && op.dc[j] != OPND_D)) {
+            set_error("vector pass %d with dot factors %d, %d, %d", op.op, op.da[j], op.db[j], op.dc[j]);
+            return MTLG_ERR_NOT_SUPPORTED;
+        }
     switch (op.op) {
 #define MTLG_VEC_PLAIN(OP) \
     case OP: k_vec<T, OP, 0><<<g, b, 0, st>>>(sv, op); break;
