@@ -155,8 +155,6 @@ struct TriFactor {
     int gnx, gny, gnz;  // gnx == 0: no grid layout
     int gns;            // entries per row (directions present): 0, 2 or 3
     int gperm;          // slot order of the directions (the reference's entry order)
-    int gdirs;          // directions present (bit d)
-    int gnsteps;        // steps per unit
     int gnsp;           // steps per unit in the layout (a multiple of kGridStepPad)
     int gnjb;           // units along y
     const void* gdata;  // S

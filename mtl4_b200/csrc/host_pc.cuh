@@ -46,7 +46,7 @@ struct TriDev {
     // grid layout (k_sweep_grid; gnx == 0: the pattern is not a grid
     // stencil): geometry as in TriFactor, per element the value source and
     // pivot row (kept until the values are filled), the values (type S)
-    int gnx = 0, gny = 0, gnz = 0, gns = 0, gperm = 0, gdirs = 0, gskew = 0, gnsteps = 0, gnsp = 0, gnjb = 0;
+    int gnx = 0, gny = 0, gnz = 0, gns = 0, gperm = 0, gnsteps = 0, gnsp = 0, gnjb = 0;
     DBuf<unsigned char> ghalo[2];      // hand-off rows between tiles for FP64 [0] / FP32 [1] vectors (all sentinel)
     long long gnent = 0;
     bool grid_indices = true;   // false: values filled straight from the matrix's CSR (no gsrc / gmul)
@@ -873,8 +873,6 @@ inline TriFactor tri_view(const TriDev& T)
         f.gnz = T.gnz;
         f.gns = T.gns;
         f.gperm = T.gperm;
-        f.gdirs = T.gdirs;
-        f.gnsteps = T.gnsteps;
         f.gnsp = T.gnsp;
         f.gnjb = T.gnjb;
         f.gdata = T.gval.p;
@@ -997,7 +995,7 @@ inline bool detect_grid(const RowLists& F, int n, bool lower, TriDev& T)
         T.gnx = std::min(n, 256);
         T.gny = (n + T.gnx - 1) / T.gnx;
         T.gnz = 1;
-        T.gns = T.gperm = T.gdirs = T.gskew = 0;
+        T.gns = T.gperm = 0;
         return true;
     }
     if (offs.size() == 1 || offs[0] != 1 || offs[1] < 2 || offs[1] > n) return false;
@@ -1065,8 +1063,6 @@ inline bool detect_grid(const RowLists& F, int n, bool lower, TriDev& T)
     T.gnz = nz;
     T.gns = ns;
     T.gperm = perm;
-    T.gdirs = ns == 3 ? 7 : 3;
-    T.gskew = 1;
     return true;
 }
 
@@ -1509,7 +1505,7 @@ inline int grid_factorize(mtlg_pc* P, bool& done)
     done = false;
     mtlg_ctx* c = P->ctx;
     const TriDev& L = P->L;
-    if (L.gnx == 0 || L.gns < 2 || !L.gskew) return MTLG_OK;
+    if (L.gnx == 0 || L.gns < 2) return MTLG_OK;
     if (L.gperm != (L.gns == 3 ? kGridFar3 : kGridFar2)) return MTLG_OK;
     const int kind = P->kind == MTLG_PC_IC0 ? kGridIC0 : kGridILU0;
     if (kind == kGridILU0 && (L.gnx < 3 || (L.gns == 3 && L.gny < 3) || (L.gns == 2 && L.gny < 2))) return MTLG_OK;
@@ -1537,8 +1533,6 @@ inline int grid_factorize(mtlg_pc* P, bool& done)
     d.L.gnz = L.gnz;
     d.L.gns = L.gns;
     d.L.gperm = L.gperm;
-    d.L.gdirs = L.gdirs;
-    d.L.gnsteps = L.gnsteps;
     d.L.gnsp = L.gnsp;
     d.L.gnjb = L.gnjb;
     d.L.gdata = lay.p;

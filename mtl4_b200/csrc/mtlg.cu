@@ -149,11 +149,12 @@ int pc_sweeps(mtlg_pc* P, const mtlg_vec* x, mtlg_vec* y)
         memset(&op, 0, sizeof op);
         op.skip = SKIP_NONE;
         op.sleep_ns = c->sweep_sleep_ns;
-        // y0 = L^{-1} x  (temp, slot 0); the chunked sweep clears y row by row
+        // y0 = L^{-1} x  (temp, slot 0).  Chunked sweeps clear y (op.reset) row
+        // by row; grid sweeps leave it, and the temp their values
         op.tasks = pl.tl.p; op.ntasks = pl.ntl; op.ticket = P->tickets.p + 2; op.which = 0;
         op.in = SLOT_X; op.out = 0; op.reset = SLOT_B;
         MTLG_TRY((launch_chunk_sweep<T, S>(c, c->stream, sv, op, pl)));
-        // y = U^{-1} y0; clears the temp again
+        // y = U^{-1} y0; a chunked sweep clears the temp again
         op.tasks = pl.tu.p; op.ntasks = pl.ntu; op.ticket = P->tickets.p + 3; op.which = 1;
         op.in = 0; op.out = SLOT_B; op.reset = 0;
         MTLG_TRY((launch_chunk_sweep<T, S>(c, c->stream, sv, op, pl)));
@@ -1108,7 +1109,7 @@ int mtlg_grid_structure(int64_t n, const int64_t* row_ptr, const int32_t* col, i
     out8[2] = T.gnz;
     out8[3] = T.gns;
     out8[4] = T.gns == 0 ? 0 : (T.gperm == (T.gns == 3 ? kGridFar3 : kGridFar2) ? 1 : 2);
-    out8[5] = T.gskew;
+    out8[5] = T.gns > 0 ? 1 : 0;
     return MTLG_OK;
 }
 

@@ -183,7 +183,7 @@ struct ChunkSweepOp {
     int ntasks;
     int* ticket;        // zero before the launch; returned to zero by the last grab
     int which;          // 0: L, 1: U
-    int in, out, reset; // vector slots (reset: SLOT_NONE or cleared to the sentinel)
+    int in, out, reset; // vector slots (reset: SLOT_NONE or cleared to the sentinel; not by grid sweeps)
     int skip;
     int sleep_ns;
     int vec_bytes;      // shared cells (chunk rows, the +0 cell, receive slots) of the largest chunk, 16-byte multiple
