@@ -61,6 +61,9 @@ constexpr int kMaxDots = 4;           // dots a fused pass can reduce at once
 constexpr int kNumVec = 16;           // workspace vectors per system
 constexpr double kRefMinGain = 0.5;  // refinement: an outer step must at least halve the FP64 residual
 constexpr int kScalarMeanRow = 12;   // SpMV auto choice: thread per row up to this mean row length
+constexpr int kDirMeanRow = 11;      // ... where x is the CG direction, formed from two vectors per entry, and
+constexpr int kDirTilesPerSm = 5;    //     the tiles are this few
+constexpr int kTwoRoundMeanRow = 7;  // ... where some CTAs run two tiles and others one
 constexpr long long kSpinLimit = 1LL << 20;  // polls before a device wait gives up (~0.5 s); default spin_limit
 
 // Tile kinds of the SpMV / vector tiling.
@@ -231,7 +234,7 @@ struct SetView {
     unsigned long long cond;     // cudaGraphConditionalHandle (0: not in a graph)
     int use_cond;
     long long spin;              // polls before a dependency wait gives up (context "spin_limit"; 0: kSpinLimit)
-    int short_rows;              // every system's rows are short and regular (csr_short_rows): SpMV by thread per row
+    int short_rows;              // every system's rows are short and regular (the least csr_short_rows): SpMV by thread per row
 };
 
 // ----------------------------------------------------------------- device helpers

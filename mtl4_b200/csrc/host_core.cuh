@@ -389,14 +389,16 @@ struct mtlg_csr {
 
 namespace mtlg {
 
-// Short, regular rows: at most kShortRow entries each and kScalarMeanRow on
-// average.  A thread per row then wins over staged tiles (FP64 7-point product
-// on 128^3: standalone 45 us against 67, with dots in a solve 77 against 106),
-// whose barriers and buffers pay off on longer or uneven rows, where a
-// thread's walk is uncoalesced.
-inline bool csr_short_rows(const mtlg_csr* A)
+// Short, regular rows: at most kShortRow entries each and kScalarMeanRow (1),
+// kDirMeanRow (2) or kTwoRoundMeanRow (3) on average; 0: others.  A thread per row then wins over
+// staged tiles (FP64 7-point product on 128^3: standalone 45 us against 67,
+// with dots in a solve 80 against 106), whose barriers and buffers pay off on
+// longer or uneven rows, where a thread's walk is uncoalesced.  Where the line
+// lies in a solve: launch_spmv.
+inline int csr_short_rows(const mtlg_csr* A)
 {
-    return !A->irregular && A->n_rows > 0 && A->nnz <= int64_t(kScalarMeanRow) * A->n_rows;
+    if (A->irregular || A->n_rows == 0 || A->nnz > int64_t(kScalarMeanRow) * A->n_rows) return 0;
+    return A->nnz <= int64_t(kTwoRoundMeanRow) * A->n_rows ? 3 : A->nnz <= int64_t(kDirMeanRow) * A->n_rows ? 2 : 1;
 }
 
 inline int ensure_f32_values(mtlg_csr* A)
@@ -442,7 +444,7 @@ inline int csr_op_set(mtlg_csr* A, SetView& sv)
     sv.err = A->misc.p + 1;
     sv.cond = 0;
     sv.use_cond = 0;
-    sv.short_rows = csr_short_rows(A) ? 1 : 0;
+    sv.short_rows = csr_short_rows(A);
     return MTLG_OK;
 }
 
@@ -625,17 +627,37 @@ inline int launch_spmv(mtlg_ctx* c, cudaStream_t st, const SetView& sv, const Sp
         MTLG_TRY(launch_spmv<T>(c, st, sv, plain, xf, asg));
         return launch_dot_ref(c, st, sv, r);
     }
-    if (sv.short_rows && op.ndot <= 2) {
+    // Thread per row or staged tiles (the same bits).  Thread per row takes rows
+    // of up to 12 entries on average (per iteration at a million rows: CG 0.65-0.95
+    // times the staged time, BiCGSTAB 0.72-0.88), but for two ranges:
+    //  - it holds two CTAs per SM, staged tiles three: between one tile for each
+    //    CTA of the two and of the three, some of its CTAs run a second tile,
+    //    which costs what the first did (CG, 75,000 rows of 8-11 random entries:
+    //    1.05-1.2 times the staged time; BiCGSTAB 1.0-1.08).  Rows of up to
+    //    kTwoRoundMeanRow entries are past it soon (110,000 rows of a 7-point
+    //    grid: 0.97-0.99) and stay;
+    //  - CG's direction costs two gathers an entry, and a row's entries past the
+    //    eight that are fetched ahead wait for theirs.  Beyond kDirMeanRow
+    //    entries that shows until there are tiles enough to hide it (11.3 random
+    //    entries, 5,000 to 40,000 rows 1.03-1.05, 110,000 rows 1.05-1.14; a band
+    //    of 12 0.96-1.01; from 150,000 rows on the band gains up to a fifth).
+    const bool dir = xf == XF_CG_P || xf == XF_CG_P_JAC;
+    const int need = dir && sv.n_tiles <= kDirTilesPerSm * c->sm_count ? 2 : 1;
+    if (sv.short_rows >= need && op.ndot <= 2) {
 #define MTLG_SHORT_ND(XF, ASG, ND) k_spmv_short<T, XF, ASG, ND><<<grid, kBlock, 0, st>>>(sv, op)
 #define MTLG_SHORT_CASE(XF, ASG)                                                                  \
     if (xf == XF && asg == ASG) {                                                                 \
         const int nd = op.fin != FIN_NONE ? op.ndot : 0;                                          \
-        const int grid = std::min(sv.n_tiles, c->sm_count * ShortShape<T, XF, ASG>::occ[nd]);     \
-        if (nd == 0) MTLG_SHORT_ND(XF, ASG, 0);                                                   \
-        else if (nd == 1) MTLG_SHORT_ND(XF, ASG, 1);                                              \
-        else MTLG_SHORT_ND(XF, ASG, 2);                                                           \
-        c->launches++;                                                                            \
-        return MTLG_OK;                                                                           \
+        const int most = c->sm_count * ShortShape<T, XF, ASG>::occ[nd];                           \
+        const int grid = std::min(sv.n_tiles, most);                                              \
+        if (sv.short_rows == 3 || sv.n_tiles <= most ||                                           \
+            sv.n_tiles > c->sm_count * SpmvShape<T, XF, ASG>::occ) {                              \
+            if (nd == 0) MTLG_SHORT_ND(XF, ASG, 0);                                               \
+            else if (nd == 1) MTLG_SHORT_ND(XF, ASG, 1);                                          \
+            else MTLG_SHORT_ND(XF, ASG, 2);                                                       \
+            c->launches++;                                                                        \
+            return MTLG_OK;                                                                       \
+        }                                                                                         \
     }
         MTLG_SPMV_VARIANTS(MTLG_SHORT_CASE)
 #undef MTLG_SHORT_CASE

@@ -262,11 +262,11 @@ inline int srv_rebuild(mtlg_server* S, int e)
     std::vector<Tile> tiles;
     std::vector<int> stb(ss.S + 1, 0);
     int maxlev = 0;
-    ss.short_rows = 1;
+    ss.short_rows = 3;
     for (int s = 0; s < ss.S; ++s) {
         if (E.slot_req[s] >= 0) {
             auto& R = *S->reqs[E.slot_req[s]];
-            if (!csr_short_rows(R.A)) ss.short_rows = 0;
+            ss.short_rows = std::min(ss.short_rows, csr_short_rows(R.A));
             plan_tiles(R.A->h_rp.data(), int(R.n), s, tiles);
             maxlev = std::max({maxlev, R.P->L.nlev, R.P->U.nlev});
         }

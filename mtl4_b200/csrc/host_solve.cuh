@@ -34,7 +34,7 @@ struct SolveSet {
     DBuf<SysDesc> desc, desc64;
     DBuf<SysState> st;
     int n_tiles = 0;
-    int short_rows = 0;   // every system's rows are short and regular
+    int short_rows = 0;   // how short and regular the systems' rows are (the least csr_short_rows)
     bool whole_tiles = false;   // the product's tiles are the vector passes': kTileRows rows each but a system's last
     DBuf<Tile> tiles;
     DBuf<int> stb;
@@ -124,10 +124,10 @@ inline int build_set(mtlg_ctx* c, SolveSet& ss)
     std::vector<int> stb(ss.S + 1, 0);
     long long maxn = 1;
     bool all_identity = true, all_jacobi = true;
-    ss.short_rows = 1;
+    ss.short_rows = 3;
     for (int s = 0; s < ss.S; ++s) {
         const SysInput& si = ss.in[s];
-        if (si.A->n_rows > 0 && !csr_short_rows(si.A)) ss.short_rows = 0;
+        if (si.A->n_rows > 0) ss.short_rows = std::min(ss.short_rows, csr_short_rows(si.A));
         plan_tiles(si.A->h_rp.data(), int(si.A->n_rows), s, tiles);
         stb[s + 1] = int(tiles.size());
         maxn = std::max<long long>(maxn, si.A->n_rows);

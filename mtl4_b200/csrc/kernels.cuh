@@ -578,10 +578,10 @@ __global__ void __launch_bounds__(kBlock, 3) k_spmv(SetView sv, SpmvOp op)
 // (SetView::short_rows): a thread takes one row of each tile straight from
 // global memory, entries 8 at a time in storage order (k_spmv's arithmetic to
 // the bit).  Bound by HBM: adjacent rows of a warp use the sectors the first
-// of them brought in, and there is no staging and no barrier per tile (FP64 BiCGSTAB product with two
-// dots on 128^3, cold caches: k_spmv 106 us, this kernel 80 us; floor 38 us at
-// 6.65 TB/s).
-// Each CTA walks a contiguous run of tiles.
+// of them brought in, and there is no staging and no barrier per tile (FP64
+// BiCGSTAB product with two dots on 128^3, cold caches: k_spmv 106 us, this
+// kernel 80 us; floor 39 us at 6.55 TB/s).  Each CTA walks a contiguous run of
+// tiles.
 template <typename T, int XF, int ASG, int ND>
 __global__ void __launch_bounds__(kBlock, 2) k_spmv_short(SetView sv, SpmvOp op)
 {
