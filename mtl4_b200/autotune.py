@@ -265,7 +265,9 @@ def tune_pc(ctx, Ad, kind: str, value=np.float32, cache: Cache | None = None, re
 def tune_vec(ctx, Ad, value=np.float64, cache: Cache | None = None, iters: int = 30, reps: int = 2,
              gpu: str | None = None):
     """Chooses vec_ctas_per_sm by timing `iters` unpreconditioned CG
-    iterations on Ad (the fused SpMV+dot and vector passes of the loop)."""
+    iterations on Ad (the fused SpMV+dot and vector passes of the loop),
+    launched one by one: a small system's one-launch CG has no such passes,
+    and a captured loop keeps the grid it was captured with."""
     from . import itl, mtl
     cache = cache or Cache()
     dt = np.dtype(value)
@@ -286,7 +288,12 @@ def tune_vec(ctx, Ad, value=np.float64, cache: Cache | None = None, iters: int =
         apply_settings(ctx, c)
         return _timed(run, reps, ctx)
 
-    choice, timings = best_of([{"vec_ctas_per_sm": v} for v in VEC_CTAS], measure)
+    loop_mode = ctx.get_tuning("loop_mode")
+    ctx.set_tuning("loop_mode", 2)
+    try:
+        choice, timings = best_of([{"vec_ctas_per_sm": v} for v in VEC_CTAS], measure)
+    finally:
+        ctx.set_tuning("loop_mode", loop_mode)
     apply_settings(ctx, choice)
     cache.put(key, {"choice": choice, "timings": timings})
     return choice, False
