@@ -147,8 +147,9 @@ int64_t mtlg_ctx_kernel_launches(mtlg_ctx* ctx);
 /* Launch-shape tuning (used by the autotuner): "sweep_blocks_per_sm"
  * (default 1), "sweep_blocks" (absolute grid of the triangular sweeps,
  * overrides the former when > 0), "sweep_sleep_ns" (poll back-off, default
- * 0), "loop_mode" (0: the Krylov loop runs as chunks of 8 iterations in
- * plain CUDA graphs, two in flight; 1: one graph with a WHILE conditional
+ * 0), "loop_mode" (0: a small CG solve without a preconditioner or with the
+ * diagonal one runs in one launch, any other Krylov loop as chunks of 8
+ * iterations in plain CUDA graphs, two in flight; 1: one graph with a WHILE conditional
  * node per solve; 2: the loop bodies launched directly, no graph -- for
  * profilers that do not see kernels inside graphs), "spmv_kernel" (standalone SpMV: 0 chooses by row
  * lengths, 1 shared-memory stream tiles, 2 row-aligned warp tasks, 3 one
@@ -181,7 +182,8 @@ int64_t mtlg_ctx_kernel_launches(mtlg_ctx* ctx);
  * triangular sweeps or factorizations gives up and the call returns
  * MTLG_ERR_TIMEOUT; 0, default: 2^20, about half a second; applies to
  * mtlg_pc_apply at once and to solves of preconditioners created
- * afterwards).
+ * afterwards; below the default CG solves do without the one launch, whose
+ * CTAs wait on one another).
  * Read-only keys for get: "sweep_max_blocks_per_sm", "sm_count". */
 int mtlg_ctx_set_tuning(mtlg_ctx* ctx, const char* key, int64_t value);
 int mtlg_ctx_get_tuning(mtlg_ctx* ctx, const char* key, int64_t* value);

@@ -14,11 +14,10 @@ Knobs and what measures them:
   sweep_cluster    CTAs per cluster of the chunked sweeps (0 automatic)
   grid_warps       compute warps per CTA of the grid sweeps (grid-stencil
                    factors; 0 automatic)                       (tune_pc)
-  sweep_sleep_ns   back-off of the sweeps' dependency polls    (tune_pc)
   vec_ctas_per_sm  CTAs per SM of the vector passes of the Krylov loops
                                                                (tune_vec)
-  sweep_blocks, sweep_sleep_ns   grid and back-off of the flat sweep kernel
-                                                               (tune_sweeps)
+  sweep_blocks, sweep_sleep_ns   grid of the flat sweep kernel, back-off of
+                   every sweep's polls                         (tune_sweeps)
 
 The chunked-sweep and vector knobs are also tuned on a batch of systems
 (tune_batch), measuring the batched solve itself.  Several knobs are searched

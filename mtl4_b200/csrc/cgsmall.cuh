@@ -7,8 +7,8 @@
 // and meet twice per iteration.  What bounds such a solve is latency: two
 // kernels an iteration cost 20 us at 65,536 rows (launch, tile metadata,
 // partials, a last CTA that gathers them), while its bytes take 1 us.
-// Measured (one B200, 256 x 256 Laplacian, FP64, diagonal): 20.4 -> 11 us an
-// iteration.
+// Measured (one B200, 256 x 256, FP64, diagonal): 20.9 -> 10.4 us an iteration;
+// other sizes at the rule that chooses it (cg_small_rows).
 //
 // A meeting: every CTA puts its tiles' partial dots into cells of a buffer
 // that is all sentinel before; CTA 0 polls the cells, adds them in

@@ -616,10 +616,13 @@ inline int run_loop_chunked(SolveSet& ss, int max_iter)
 // does not apply: one system, no or diagonal preconditioner, short regular
 // rows, whole 256-row product tiles (they are the vector passes' tiles then,
 // so the dots' partials are the same; tiles that kTileNnz entries cut short
-// add the same products up in another grouping), and few enough rows that all
-// run at once.  Two kernels an iteration win again only where a pass is long against
-// its launch (beyond these sizes).  Not in the reference's summation order,
-// whose dots are whole-vector chains.
+// add the same products up in another grouping), and at most four rows per
+// thread of one CTA per SM.  Per iteration, one launch / two kernels (FP64,
+// diagonal, one B200): 1,023 rows 8.5 / 19.8 us, 37,636 (one row per thread)
+// 10.8 / 20.1, 75,624 (two) 9.7 / 21.1, 78,400 (four) 16.2 / 22.1, 148,877 of a
+// 7-point grid 19.2 / 24.2: the gap, which is the launches, narrows with the
+// rows.  Not in the reference's summation order, whose dots are whole-vector
+// chains.
 template <typename T>
 inline int cg_small_rows(const SolveSet& ss)
 {
@@ -645,8 +648,8 @@ inline int run_cg_small(SolveSet& ss, int rows, bool& ran)
 }
 
 // Runs the loop until no system is running.  Default: one launch for small CG
-// solves (run_cg_small), else chunked plain graphs (run_loop_chunked).  loop_mode 1: one graph with a WHILE conditional node,
-// one launch per solve.  If a graph cannot be built, or under loop_mode 2
+// solves (run_cg_small), else chunked plain graphs (run_loop_chunked).
+// loop_mode 1: one graph with a WHILE conditional node, one launch per solve.  If a graph cannot be built, or under loop_mode 2
 // (for profilers that do not see kernels inside graphs), the body is
 // launched directly from the host, 8 at a time.
 template <typename T>

@@ -971,7 +971,7 @@ constexpr int kVecGroup = 4;   // tiles a vector-pass CTA works on at once (one 
 // the pass's dots; a group's are reduced together (warp_sums), and the warps'
 // sums meet in shared memory only every kPartTiles tiles, so the streams of
 // loads run on (FP64 BiCGSTAB x / r pass on 128^3: 84 us with a block
-// reduction of 16 values per group, 57 us so; floor 20 us at 6.65 TB/s).
+// reduction of 16 values per group, 57 us so; floor 20 us at 6.55 TB/s).
 template <typename T, int OP, int ND>
 __global__ void __launch_bounds__(kBlock, 2) k_vec(SetView sv, VecOp op)
 {
