@@ -195,10 +195,13 @@ __device__ __forceinline__ void grid_acquire() { asm volatile("fence.acq_rel.cta
 // (recorded as a timeout), or when another wait has expired.  Decided by all
 // lanes together, every lane having counted the same polls: the waits below
 // and what follows them use warp-wide votes.  A wait of more than kGridQuick
-// polls (0.1 ms in shared memory) naps between them: it leaves the issue slots
-// to the others, and the default limit stays about half a second whatever a
-// poll costs (2^20 polls of shared memory alone: some 40 ms).
-constexpr long long kGridQuick = 4096;
+// polls (some 3 ms in shared memory, longer than the chain of a wave of tiles
+// takes to come by) naps between them: it leaves the issue slots to the others,
+// and the default limit stays about half a second whatever a poll costs (2^20
+// polls of shared memory alone: some 40 ms).  Napping from 4,096 polls on found
+// a waiting tile's rows late (FP64, lines of 2 rows, 782 tiles in a chain:
+// applies of 16.8 ms instead of 16.1).
+constexpr long long kGridQuick = 1 << 16;
 __device__ __forceinline__ bool grid_give_up(long long& spins, int* err, long long lim)
 {
     const bool over = ++spins > (lim > 0 ? lim : kSpinLimit);
